@@ -149,6 +149,9 @@ void release_workspace(Workspace &w)
     if (w.order2) cudaFree(w.order2);
     if (w.wc_rows) cudaFree(w.wc_rows);
     if (w.wc_defer) cudaFree(w.wc_defer);
+    if (w.pk_defer) cudaFree(w.pk_defer);
+    if (w.pk_q) cudaFree(w.pk_q);
+    if (w.tb_kind) cudaFree(w.tb_kind);
     if (w.aux) cudaStreamDestroy(w.aux);
     if (w.queue) cudaFree(w.queue);
     if (w.fork) cudaEventDestroy(w.fork);
@@ -233,18 +236,120 @@ static int ensure_order_buffers(Workspace &ws, size_t n)
     return GB_OK;
 }
 
-int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p, cudaStream_t s)
+static int pk_class_of(uint32_t qlen)
 {
-    if (b.n <= 0) return GB_ERR_ARG;
+    const uint32_t words = (qlen + 7) >> 3;
+    int c = 0;
+    while (words < PK_CLASS_WORDS[c]) c++;
+    return c;
+}
+
+/* Whether the packed kernels take this batch, and with what shapes.  They run
+ * LOCAL, GLOBAL and target-tail SEMI_GLOBAL pairs of every length: at 150 bp
+ * and 250-5000 bp they do two cells per instruction where the one-thread and
+ * warp-cooperative kernels do one, and in batches too small to fill the chip
+ * with a thread per pair they spread each pair over lanes.  Kept off: second
+ * best (its running-maximum rule is per cell), SEMI_GLOBAL tracebacks, scores
+ * beyond pk_scores_ok, and the plain form (persistent 0). */
+static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p, int sms)
+{
+    const Settings &st = settings();
+    const bool algo_ok = cfg.algo == LOCAL_ || cfg.algo == GLOBAL_ ||
+                         (cfg.algo == SEMI_GLOBAL_ && cfg.tail == TARGET_ && cfg.start != WITH_TB_);
+    if (!algo_ok || !st.persistent || (cfg.second && cfg.algo != GLOBAL_) || !pk_scores_ok(cfg.algo, cfg.sc))
+        return GB_OK;
+    struct {
+        int n = 0;
+        uint32_t max_q = 0, max_t = 0, max_min = 0;
+        PkSample sample;
+    } cl[PK_CLASSES];
+    uint32_t min_q = 0xFFFFFFFFu, max_q = 0;
+    const int stride = std::max(1, b.n / 1024);
+    for (int i = 0, next = 0; i < b.n; i++) {
+        const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
+        auto &c = cl[pk_class_of(ql)];
+        c.n++;
+        c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl), c.max_min = std::max(c.max_min, std::min(ql, tl));
+        min_q = std::min(min_q, ql), max_q = std::max(max_q, ql);
+        if (i == next) {
+            next += stride;
+            PkSample &sm = c.sample;
+            if (sm.n < 256) sm.qw[sm.n] = (int)((ql + 7) >> 3), sm.tw[sm.n] = (int)((tl + 7) >> 3), sm.n++;
+        }
+    }
+    /* an unordered batch is one class: equal lengths, or too few pairs for the order to matter */
+    const bool order = b.n >= st.min_order_pairs || (b.n > 64 && st.min_order_pairs <= (1 << 29) && max_q > min_q + min_q / 2);
+    if (!order) {
+        auto &z = cl[0];
+        for (int c = 1; c < PK_CLASSES; c++) {
+            z.n += cl[c].n;
+            z.max_q = std::max(z.max_q, cl[c].max_q), z.max_t = std::max(z.max_t, cl[c].max_t);
+            z.max_min = std::max(z.max_min, cl[c].max_min);
+            for (int k = 0; k < cl[c].sample.n && z.sample.n < 256; k++, z.sample.n++)
+                z.sample.qw[z.sample.n] = cl[c].sample.qw[k], z.sample.tw[z.sample.n] = cl[c].sample.tw[k];
+            cl[c].n = 0;
+        }
+    }
+    p.pk_wc = false;
+    for (int c = 0; c < PK_CLASSES; c++) {
+        if (cl[c].n == 0) continue;
+        if (!pk_fits(cfg.algo, cfg.sc, cl[c].max_q, cl[c].max_t, cl[c].max_min)) {
+            if (c > 0 || !order) return GB_OK;
+            p.pk_wc = true;
+            continue;
+        }
+        if (cl[c].sample.n == 0) {
+            cl[c].sample.n = 1;
+            cl[c].sample.qw[0] = (int)((cl[c].max_q + 7) >> 3), cl[c].sample.tw[0] = (int)((cl[c].max_t + 7) >> 3);
+        }
+        const int start = cfg.algo == GLOBAL_ && cfg.start == WITH_START_ ? WITHOUT_START_ : cfg.start;
+        const int forced = st.wc_group >= 64 ? 32 : st.wc_group;
+        p.pk_class[c].max_q = cl[c].max_q;
+        p.pk_class[c].fast = pk_plan(cfg.algo, start, true, cl[c].n, cl[c].max_q, cl[c].sample, sms, forced);
+        p.pk_class[c].cmp = pk_plan(cfg.algo, start, false, std::min(cl[c].n, 32 * sms), cl[c].max_q, cl[c].sample, sms, 0);
+        if (p.pk_class[c].fast.group == 0 || p.pk_class[c].cmp.group == 0) return GB_OK;
+    }
+    if (grow((void **)&ws.pk_defer, &ws.pk_defer_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
+    if (!ws.pk_q && dev_malloc((void **)&ws.pk_q, PK_QUEUE_WORDS * 4) != cudaSuccess) {
+        cudaGetLastError();
+        return GB_ERR_ALLOC;
+    }
+    p.pkc = pk_const(cfg.algo, cfg.sc);
+    p.pk_fill = 16 * sms;
+    p.order_on = order;
+    p.pk = true;
+    return GB_OK;
+}
+
+/* pairs [p0, p1) of each class (one class when the batch is not ordered) */
+static void count_pk_classes(const Plan &p, const DevBatch &b, int p0, int p1, int *n)
+{
+    if (!p.order_on) {
+        n[0] = p1 - p0;
+        return;
+    }
+    for (int i = p0; i < p1; i++) n[pk_class_of(b.h_q_len[i])]++;
+}
+
+static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p,
+                           cudaStream_t s)
+{
     const Settings &st = settings();
     p = Plan();
     p.block = st.block;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (packed) {
+        const int rc = plan_pk(cfg, b, ws, p, sms);
+        if (rc != GB_OK) return rc;
+    }
 
     /* split: long LOCAL/GLOBAL (and target-tail SEMI_GLOBAL) pairs go warp-cooperative */
     bool wc_algo = cfg.algo == LOCAL_ || cfg.algo == GLOBAL_ || (cfg.algo == SEMI_GLOBAL_ && cfg.tail == TARGET_);
     /* target-tail SEMI_GLOBAL WITH_TB (the extension) runs one pair per thread */
     const bool semi_tb = cfg.algo == SEMI_GLOBAL_ && cfg.start == WITH_TB_ && cfg.tail == TARGET_;
-    if (semi_tb) wc_algo = false;
+    if (semi_tb || (p.pk && !p.pk_wc)) wc_algo = false;
     if (wc_algo && cfg.start != WITHOUT_START_ && cfg.sc.match > 0) {
         /* start passes and tracebacks of pairs whose scores can leave the
          * 16-bit row buffer (match * min(qlen, tlen) >= 2^15) stay on the
@@ -261,8 +366,9 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
      * group's ring reader must trail its writer) */
     const int min_words = std::max(st.wc_min_qregs, st.wc_group > 0 ? st.wc_group : 8);
     p.wc_min_q = (uint32_t)min_words * 8 - 7;
-    for (int i = 0; i < b.n; i++) {
+    for (int i = 0; i < b.n && (!p.pk || p.pk_wc); i++) {
         const uint32_t ql = b.h_q_len[i];
+        if (p.pk && ql < big_q) continue; /* the packed kernels' */
         if (wc_algo && ql >= p.wc_min_q) {
             nlong++;
             if (ql >= big_q) {
@@ -312,7 +418,10 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
             if (grow((void **)&ws.wc_defer, &ws.wc_defer_cap, (size_t)nlong, 4) != GB_OK) return GB_ERR_ALLOC;
         }
     }
-    if (!p.use_wc) {
+    if (p.pk_wc && !p.use_wc) return plan_batch_with(false, cfg, b, o, ws, p, s); /* no kernel for class 0 */
+    if (p.pk) {
+        max_q_short = 0;
+    } else if (!p.use_wc) {
         max_q_short = std::max({max_q_short, max_q_long, max_q_big});
         nlong = 0, nbig = 0;
     }
@@ -357,10 +466,9 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
     auto cols_of = [&](uint32_t q) {
         return cfg.algo == KSW_ ? 2 * ((int)q + 2) : (int)((q + 7) & ~7u);
     };
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if ((size_t)std::max(cols, 8) * p.block * 4 <= smem_limit) {
+    if (p.pk) {
+        /* no one-thread launch */
+    } else if ((size_t)std::max(cols, 8) * p.block * 4 <= smem_limit) {
         a.smem_cols = std::max(cols, 8);
     } else {
         /* the longest query does not leave room for shared-memory rows: split
@@ -401,7 +509,7 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
             a.scratch_cols = (uint32_t)cols;
         }
     }
-    if (p.use_wc && !ws.aux) {
+    if ((p.use_wc || p.pk) && !ws.aux) {
         /* the warp-cooperative kernels run on the auxiliary stream: with the
          * launch stream's priority, so a caller's prioritised batch keeps it */
         int prio = 0;
@@ -421,7 +529,7 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
     /* SEMI_GLOBAL WITH_TB with another tail returns the reference's outputs: the forward pass alone */
     p.start = (cfg.algo == SEMI_GLOBAL_ && cfg.start == WITH_TB_ && !semi_tb) ? WITHOUT_START_ : cfg.start;
     p.second = cfg.second && (cfg.algo == LOCAL_ || cfg.algo == SEMI_GLOBAL_);
-    p.split_start = st.split_start && p.start == WITH_START_ && (cfg.algo == LOCAL_ || cfg.algo == SEMI_GLOBAL_) &&
+    p.split_start = !p.pk && st.split_start && p.start == WITH_START_ && (cfg.algo == LOCAL_ || cfg.algo == SEMI_GLOBAL_) &&
                     b.n >= st.min_order_pairs && o.score && o.q_end && o.t_end;
     if (p.split_start) {
         if (grow((void **)&ws.order2, &ws.order2_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
@@ -435,7 +543,12 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
         p.cut = {0, b.n};
         p.nlong = {nlong};
         p.nbig = {nbig};
-        p.order_on = p.use_wc || b.n >= st.min_order_pairs;
+        if (p.pk) {
+            p.pk_n.assign(PK_CLASSES, 0);
+            count_pk_classes(p, b, 0, b.n, p.pk_n.data());
+        } else {
+            p.order_on = p.use_wc || b.n >= st.min_order_pairs;
+        }
         if (p.order_on && ensure_order_buffers(ws, (size_t)b.n) != GB_OK) return GB_ERR_ALLOC;
         return GB_OK;
     }
@@ -496,11 +609,22 @@ int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace 
             }
         p.nlong.push_back(nl);
         p.nbig.push_back(nb);
+        if (p.pk) {
+            p.pk_n.resize(p.pk_n.size() + PK_CLASSES, 0);
+            count_pk_classes(p, b, p0, p1, p.pk_n.data() + p.pk_n.size() - PK_CLASSES);
+        }
         max_chunk = std::max(max_chunk, (size_t)(p1 - p0));
     }
-    p.order_on = p.use_wc || b.n >= st.min_order_pairs;
+    if (!p.pk) p.order_on = p.use_wc || b.n >= st.min_order_pairs;
+    if (p.pk && grow((void **)&ws.tb_kind, &ws.tb_kind_cap, max_chunk, 1) != GB_OK) return GB_ERR_ALLOC;
     if (p.order_on && ensure_order_buffers(ws, max_chunk) != GB_OK) return GB_ERR_ALLOC;
     return GB_OK;
+}
+
+int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p, cudaStream_t s)
+{
+    if (b.n <= 0) return GB_ERR_ARG;
+    return plan_batch_with(true, cfg, b, o, ws, p, s);
 }
 
 /* The one-thread launch(es) for DpArgs a: with two length tiers, the short
@@ -586,6 +710,73 @@ static int launch_dp_split(int algo, int start, bool second, const Plan &p, DpAr
     }
     a.order = order;
     return launch_one_thread(algo, start, second, p, a, ws, s);
+}
+
+/* DP over pairs [0, a.n) on the packed kernels, class by class (contiguous
+ * ranges of `order`; without one, every pair is class 0's).  With warps enough
+ * to fill the GPU the first class with pairs -- the longest queries, with the
+ * longest sweeps -- runs on the auxiliary stream beside the others (200k mixed
+ * LOCAL pairs: 30.6 against 34 ms one after another).  A smaller batch runs on
+ * one stream, classes of the same shape in one launch: its one-warp blocks
+ * from two streams at once landed on few SMs (1,000 pairs of 250-2,000 bp:
+ * 6.0 against 3.2 ms). */
+static int launch_pk(const RunCfg &cfg, const Plan &p, DpArgs a, const uint32_t *order, const int *pk_n, Workspace &ws,
+                     cudaStream_t s)
+{
+    GB_CUDA(cudaMemsetAsync(ws.pk_q, 0, PK_QUEUE_WORDS * 4, s));
+    a.tb_kind = ws.tb_kind;
+    if (p.tb && p.pk_wc) GB_CUDA(cudaMemsetAsync(ws.tb_kind, 0, (size_t)a.n, s));
+    int used = 0;
+    long warps = 0;
+    for (int c = 0; c < PK_CLASSES; c++) {
+        if (pk_n[c] == 0) continue;
+        used++;
+        warps += (c == 0 && p.pk_wc) ? p.pk_fill : (long)p.pk_class[c].fast.blocks * p.pk_class[c].fast.warps;
+    }
+    const bool full = warps >= p.pk_fill;
+    const bool fork = used > 1 && full;
+    if (fork) {
+        GB_CUDA(cudaEventRecord(ws.fork, s));
+        GB_CUDA(cudaStreamWaitEvent(ws.aux, ws.fork, 0));
+    }
+    const int start = cfg.algo == GLOBAL_ && p.start == WITH_START_ ? WITHOUT_START_ : p.start;
+    bool first = true;
+    for (int c = 0, at = 0; c < PK_CLASSES;) {
+        if (pk_n[c] == 0) {
+            c++;
+            continue;
+        }
+        cudaStream_t on = first && fork ? ws.aux : s;
+        first = false;
+        int n = pk_n[c];
+        timing_mark(K_DP, true, on);
+        if (c == 0 && p.pk_wc) {
+            GB_CUDA(launch_dp_wc(cfg.algo, p.start, p.second, a, order, n, p.mq8_big, p.mt8_big, p.wc_big, ws.wc_rows,
+                                 ws.wc_defer, ws.queue + 12, ws.queue + 16, on));
+            c++;
+        } else {
+            const auto &k = p.pk_class[c];
+            WcLaunch fast = k.fast, cmp = k.cmp;
+            int next = c + 1;
+            for (; !full && next < PK_CLASSES; next++) {
+                const WcLaunch &f = p.pk_class[next].fast;
+                if (pk_n[next] == 0) continue;
+                if (f.group != fast.group || f.warps != fast.warps) break;
+                n += pk_n[next];
+                fast.blocks += f.blocks, cmp.blocks += p.pk_class[next].cmp.blocks;
+            }
+            GB_CUDA(launch_dp_pk(cfg.algo, start, a, p.pkc, order ? order + at : nullptr, n, k.max_q, fast, cmp,
+                                 ws.pk_defer + at, ws.pk_q + 4 * c, on));
+            c = next;
+        }
+        timing_mark(K_DP, false, on);
+        at += n;
+    }
+    if (fork) {
+        GB_CUDA(cudaEventRecord(ws.join, ws.aux));
+        GB_CUDA(cudaStreamWaitEvent(s, ws.join, 0));
+    }
+    return GB_OK;
 }
 
 /* ksw: every pair (in `order`, or 0..n-1) to the warp-per-pair kernel --
@@ -682,6 +873,7 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
             if (rc != GB_OK) return rc;
             ord = ws.order;
         }
+        if (p.pk) return launch_pk(cfg, p, p.a, ord, p.pk_n.data(), ws, s);
         if (p.ksw_slots[0] > 0) return launch_ksw_split(cfg, b, p, ord, b.n, ws, s);
         return launch_dp_split(cfg.algo, p.start, p.second, p, p.a, ord, ord ? p.nlong[0] : 0, ord ? p.nbig[0] : 0,
                                ws, s);
@@ -703,8 +895,9 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
             if (rc != GB_OK) return rc;
             ord = ws.order;
         }
-        const int rc = launch_dp_split(cfg.algo, p.start, p.second, p, ca, ord, ord ? p.nlong[c] : 0,
-                                       ord ? p.nbig[c] : 0, ws, s);
+        const int rc = p.pk ? launch_pk(cfg, p, ca, ord, p.pk_n.data() + PK_CLASSES * c, ws, s)
+                            : launch_dp_split(cfg.algo, p.start, p.second, p, ca, ord, ord ? p.nlong[c] : 0,
+                                              ord ? p.nbig[c] : 0, ws, s);
         if (rc != GB_OK) return rc;
         TbArgs t{};
         t.tb = ws.tb, t.tb_off = ws.d_tb_off + p0;
@@ -715,7 +908,13 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
         t.n_cigar = o.n_cigar ? o.n_cigar + p0 : nullptr;
         t.n = ca.n, t.algo = cfg.algo, t.sc = cfg.sc, t.head = cfg.head;
         timing_mark(K_TB, true, s);
-        GB_CUDA(launch_traceback(t, s));
+        if (p.pk) {
+            t.kind = ws.tb_kind, t.order = ord;
+            t.pq = b.pq, t.pt = b.pt, t.t_off = ca.t_off;
+            t.c0 = p.pkc.c0, t.pa = p.pkc.a, t.pb = p.pkc.b;
+            GB_CUDA(launch_traceback_points(t, s));
+        }
+        if (!p.pk || p.pk_wc) GB_CUDA(launch_traceback(t, s));
         timing_mark(K_TB, false, s);
     }
     return GB_OK;

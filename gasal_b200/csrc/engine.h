@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "gb_internal.h"
+#include "dp_pk.h"
 #include "gasal_b200_capi.h"
 
 namespace gb {
@@ -69,6 +70,11 @@ struct Workspace {
     size_t wc_rows_cap = 0;
     uint32_t *wc_defer = nullptr; /* pairs the table-scoring warp-cooperative launch leaves to compare scoring */
     size_t wc_defer_cap = 0;
+    uint32_t *pk_defer = nullptr; /* pairs the packed table-scoring launches leave to the compare-scoring ones */
+    size_t pk_defer_cap = 0;
+    uint32_t *pk_q = nullptr;    /* PK_QUEUE_WORDS counters of the packed launches */
+    uint8_t *tb_kind = nullptr;  /* per pair of a traceback chunk: 1 = boundary checkpoints, 0 = direction tiles */
+    size_t tb_kind_cap = 0;
     uint32_t *order2 = nullptr;  /* visiting order of the separate start passes */
     size_t order2_cap = 0;
     uint32_t *bins = nullptr;    /* order_bins() class counters */
@@ -95,6 +101,13 @@ void mix_release_all();
 /* the band entry points' per-stream workspaces (band_api.cu) */
 void band_release_all();
 
+/* The packed kernels run one pair of launches per class of query lengths, a
+ * contiguous range of the length order; class c takes queries of at least
+ * PK_CLASS_WORDS[c] words (and fewer than class c-1's). */
+constexpr int PK_CLASSES = 5;
+constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {ORDER_CAP_WORDS, 64, 32, 16, 0};
+constexpr int PK_QUEUE_WORDS = 4 * PK_CLASSES;
+
 /* The decisions and allocations for one batch (plan_batch), so that
  * enqueue_batch issues stream operations only -- capturable into a graph. */
 struct Plan {
@@ -117,6 +130,15 @@ struct Plan {
     bool split_start = false; /* one-thread start passes as a second launch (order2) */
     int fb_blocks = 0;      /* grid of the one-thread ksw launch for handed-back pairs (scratch rows) */
     DpArgs a{};
+    bool pk = false;        /* the packed kernels (dp_pk.cuh) run every class but pk_wc's */
+    bool pk_wc = false;     /* ... class 0's values leave their range: it runs warp-cooperative (wc_big) */
+    PkConst pkc{};
+    struct {
+        uint32_t max_q = 0;
+        WcLaunch fast, cmp;
+    } pk_class[PK_CLASSES];
+    long pk_fill = 0;       /* warps that fill the GPU */
+    std::vector<int> pk_n;  /* per range, per class: its pairs */
     std::vector<int> cut;   /* pair ranges [cut[c], cut[c+1]) run one after another */
     std::vector<int> nlong; /* per range: pairs on the warp-cooperative kernel */
     std::vector<int> nbig;  /* per range: of those, the leading ORDER_CAP_WORDS+ word ones */
@@ -131,11 +153,14 @@ int enqueue_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspa
                   cudaStream_t s);
 int run_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, cudaStream_t s);
 
-/* Traceback tiles of one pair, in uint4 units (two spare tile rows). */
+/* Traceback storage of one pair, in uint4 units: direction tiles (two spare
+ * tile rows), or the packed kernels' checkpoints -- a word per column every
+ * 16 rows and per row every 16 columns. */
 inline uint64_t tb_tiles(uint32_t qlen, uint32_t tlen)
 {
     const uint64_t qr = (qlen + 7) >> 3, tr = (tlen + 7) >> 3;
-    return (tr + 2) * 2 * qr;
+    const uint64_t tiles = (tr + 2) * 2 * qr, points = ((tr + 1) / 2 * qr + (qr + 1) / 2 * tr) * 2;
+    return tiles > points ? tiles : points;
 }
 
 /* Process-wide settings (set through the C ABI). */

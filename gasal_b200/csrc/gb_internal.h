@@ -57,6 +57,8 @@ struct DpArgs {
                                            one slot of scratch_cols words per lane group of the grid */
     int32_t *max_off;                   /* unbanded ksw: largest |column - row| of the cells where the
                                            running maximum rose (ksw_extend2's max_off), or null */
+    uint8_t *tb_kind;                   /* per pair: 1 when its traceback storage holds boundary
+                                           checkpoints (dp_pk.cuh) instead of direction tiles */
     uint32_t *defer, *ndefer;           /* warp-cooperative table-scoring launch: pairs it leaves to the
                                            compare-scoring launch, and their count */
 };
@@ -81,6 +83,10 @@ struct TbArgs {
     int32_t algo;
     Scores sc;
     int32_t head;                       /* SEMI_GLOBAL: which leading bases are free */
+    const uint8_t *kind;                /* per pair: 1 = checkpoints (traceback_points_kernel) */
+    const uint32_t *order;              /* visiting order of the checkpoint walks, or null */
+    const uint32_t *pq, *pt, *t_off;    /* packed words, for recomputing blocks */
+    int32_t c0, pa, pb;                 /* the packed kernels' offsets (PkConst) */
 };
 
 /* ---- launchers (stream-ordered, no allocation) ---- */
@@ -91,6 +97,8 @@ cudaError_t launch_revcomp(uint32_t *pq, uint32_t *pt, const uint32_t *q_off, co
 cudaError_t launch_dp(int algo, int start, bool second, const DpArgs &a, int block, int max_q8,
                       cudaStream_t s);
 cudaError_t launch_traceback(const TbArgs &a, cudaStream_t s);
+/* the pairs whose kind is 1 (LOCAL, GLOBAL): walks over recomputed blocks */
+cudaError_t launch_traceback_points(const TbArgs &a, cudaStream_t s);
 
 /* Lets a kernel use the most dynamic shared memory the device gives a block
  * (set once per kernel and device).  Kernels launched with different sizes

@@ -101,7 +101,7 @@ __device__ uint32_t semi_walk(const uint4 *tb, int q8, int i, int j, int head, u
 __global__ void __launch_bounds__(128) traceback_kernel(TbArgs a)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n) return;
+    if (p >= a.n || (a.kind && a.kind[p])) return;
     const int qlen = (int)a.q_len[p], tlen = (int)a.t_len[p];
     uint32_t n_ops = 0;
     if (a.algo == SEMI_GLOBAL_) {
@@ -181,6 +181,172 @@ __global__ void __launch_bounds__(128) traceback_kernel(TbArgs a)
         if (a.q_start) a.q_start[p] = 0;
     }
     if (a.n_cigar) a.n_cigar[p] = n_ops;
+}
+
+/* Traceback from the packed kernels' checkpoints (LOCAL, GLOBAL).  The
+ * forward sweep writes no direction code per cell (a dozen integer operations
+ * on top of a cell's five to nine): it leaves H and E entering every 16th row
+ * and D and F entering every 16th column (0.5 B per cell, as the tiles), and
+ * the walk recomputes the 16 x 16 blocks its path crosses, each from its own
+ * exact borders -- about 32 cells per base of the path instead of a code for
+ * every cell of the matrix.  One thread per pair, in length order; the warp
+ * alternates between recomputing every lane's block and walking every lane to
+ * its block's edge, so the lanes stay together. */
+constexpr int TBP_THREADS = 64;
+
+template <bool LOC> __global__ void __launch_bounds__(TBP_THREADS) traceback_points_kernel(TbArgs a)
+{
+    __shared__ uint2 nibs[16][TBP_THREADS];
+    const int slot = blockIdx.x * TBP_THREADS + threadIdx.x;
+    const int tid = threadIdx.x;
+    int p = 0;
+    bool have = slot < a.n;
+    if (have) {
+        p = a.order ? (int)a.order[slot] : slot;
+        have = a.kind[p] != 0;
+    }
+    int qlen = 0, tlen = 0;
+    if (have) qlen = (int)a.q_len[p], tlen = (int)a.t_len[p];
+    const bool real = have && qlen > 0 && tlen > 0;
+    const int qregs = (qlen + 7) >> 3, tregs = (tlen + 7) >> 3, q8 = qregs << 3, t8 = tregs << 3;
+    const uint32_t *tops = nullptr, *lefts = nullptr, *qw = nullptr, *tw = nullptr;
+    int i = -1, j = -1, total = 0;
+    uint8_t *out = nullptr;
+    uint32_t room = 0;
+    if (real) {
+        tops = reinterpret_cast<const uint32_t *>(a.tb + a.tb_off[p]);
+        lefts = tops + (size_t)((tregs + 1) >> 1) * q8;
+        qw = a.pq + (a.q_off[p] >> 3), tw = a.pt + (a.t_off[p] >> 3);
+        if (LOC) i = a.t_end[p], j = a.q_end[p], total = a.score[p];
+        else i = tlen, j = qlen;
+        out = a.cigar + a.q_off[p];
+        room = a.q_off[p] < a.cigar_bytes ? a.cigar_bytes - a.q_off[p] : 0u;
+    }
+    const Scores sc = a.sc;
+    uint32_t n_ops = 0, prev_op = 0, op_fill = 0;
+    int op_select = 3, op_shift = 0, count = 0, curr = 0;
+    bool done = !real;
+    while (__any_sync(0xFFFFFFFFu, !done && i >= 0 && j >= 0)) {
+        const bool on = !done && i >= 0 && j >= 0;
+        const int bi = i >> 4, bj = j >> 4;
+        const bool in = on && i < t8 && j < q8;
+        /* recompute the block's rows down to the walk's */
+        if (__any_sync(0xFFFFFFFFu, in)) {
+            int Hup[16], E[16];
+            uint32_t qa = 0, qb = 0;
+            const int rows = in ? (i & 15) + 1 : 0;
+            if (in) {
+                const uint4 *t4 = reinterpret_cast<const uint4 *>(tops + (size_t)bi * q8 + (bj << 4));
+                qa = qw[2 * bj];
+                const bool two = 2 * bj + 1 < qregs;
+                if (two) qb = qw[2 * bj + 1];
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    const uint4 v = g < 2 || two ? t4[g] : make_uint4(0, 0, 0, 0);
+                    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int c = 4 * g + u, off = a.c0 + a.pb * ((c & 7) + 1);
+                        Hup[c] = (int)(x[u] & 0xFFFFu) - off;
+                        E[c] = (int)(x[u] >> 16) - off - a.pa;
+                    }
+                }
+            }
+            const uint32_t *lf = lefts + (size_t)bj * t8 + (bi << 4);
+            for (int r = 0; r < 16; r++) {
+                if (!__any_sync(0xFFFFFFFFu, r < rows)) break;
+                if (r < rows) {
+                    const uint32_t l = lf[r];
+                    const int off = a.c0 + a.pa * (r & 7);
+                    int diag = (int)(l & 0xFFFFu) - off, F = (int)(l >> 16) - off - a.pa - a.pb;
+                    const uint32_t tword = tw[2 * bi + (r >> 3)];
+                    const uint32_t tc = (tword >> (28 - 4 * (r & 7))) & 15u;
+                    uint32_t lo = 0, hi = 0;
+#pragma unroll
+                    for (int c = 0; c < 16; c++) {
+                        const uint32_t qc = ((c < 8 ? qa : qb) >> (28 - 4 * (c & 7))) & 15u;
+                        int s = qc == tc ? sc.match : -sc.mismatch;
+                        if (LOC && (qc == 14u || tc == 14u)) s = 0;
+                        const int M = diag + s;
+                        int H = max(max(M, F), E[c]);
+                        if (LOC) H = max(H, 0);
+                        uint32_t d = (H == M) ? (M >= diag ? 0u : 1u) : (H == F ? 3u : 2u);
+                        const int t0 = M - sc.oe;
+                        d |= t0 > F - sc.e ? 0u : 8u;
+                        d |= t0 > E[c] - sc.e ? 0u : 4u;
+                        if (c < 8) lo |= d << (4 * c);
+                        else hi |= d << (4 * (c - 8));
+                        F = max(F - sc.e, t0);
+                        E[c] = max(E[c] - sc.e, t0);
+                        diag = Hup[c];
+                        Hup[c] = H;
+                    }
+                    nibs[r][tid] = make_uint2(lo, hi);
+                }
+            }
+        }
+        /* walk to the block's edge; a cell past the matrix (GLOBAL's first)
+         * reads 0, and the block that its successor lies in comes next */
+        bool go = on;
+        while (go) {
+            uint32_t nib = 0;
+            if (in) {
+                const uint2 w = nibs[i & 15][tid];
+                nib = ((j & 8 ? w.y : w.x) >> (4 * (j & 7))) & 15u;
+            }
+            const uint32_t op = (nib >> op_shift) & (uint32_t)op_select;
+            op_fill = (op == 0 || op_select == 3) ? op : (uint32_t)op_shift;
+            const bool normal = op == 0 || (op == 1 && op_select == 3);
+            op_shift = normal ? 0 : ((op == 2 || op == 3) ? (int)op : op_shift);
+            op_select = normal ? 3 : 1;
+            if (count < 63 && op_fill == prev_op) {
+                count++;
+            } else {
+                if (count > 0) {
+                    if (n_ops < room) out[n_ops] = (uint8_t)(prev_op | ((uint32_t)count << 2));
+                    n_ops++;
+                }
+                count = 1;
+            }
+            if (LOC) {
+                const bool gap = (op_fill == 2 || op_fill == 3);
+                curr += (gap && prev_op != op_fill) ? -sc.oe : (gap ? -sc.e : (op_fill == 1 ? -sc.mismatch : sc.match));
+                if (curr == total) {
+                    done = true;
+                    break;
+                }
+            }
+            prev_op = op_fill;
+            if (op_fill == 0 || op_fill == 1 || op_fill == 2) i--;
+            if (op_fill == 0 || op_fill == 1 || op_fill == 3) j--;
+            go = in && i >= 0 && j >= 0 && (i >> 4) == bi && (j >> 4) == bj;
+        }
+    }
+    if (!have) return;
+    if (real) {
+        if (n_ops < room) out[n_ops] = (uint8_t)(prev_op | ((uint32_t)count << 2));
+        n_ops++;
+        if (!LOC) {
+            for (; i >= 0; i -= 63, n_ops++)
+                if (n_ops < room) out[n_ops] = (uint8_t)(2u | ((uint32_t)min(i + 1, 63) << 2));
+            for (; j >= 0; j -= 63, n_ops++)
+                if (n_ops < room) out[n_ops] = (uint8_t)(3u | ((uint32_t)min(j + 1, 63) << 2));
+        }
+    }
+    if (LOC) {
+        if (a.t_start) a.t_start[p] = real ? i : 0;
+        if (a.q_start) a.q_start[p] = real ? j : 0;
+    }
+    if (a.n_cigar) a.n_cigar[p] = n_ops;
+}
+
+cudaError_t launch_traceback_points(const TbArgs &a, cudaStream_t s)
+{
+    if (a.n <= 0) return cudaSuccess;
+    const int blocks = (a.n + TBP_THREADS - 1) / TBP_THREADS;
+    if (a.algo == LOCAL_) traceback_points_kernel<true><<<blocks, TBP_THREADS, 0, s>>>(a);
+    else traceback_points_kernel<false><<<blocks, TBP_THREADS, 0, s>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_traceback(const TbArgs &a, cudaStream_t s)
