@@ -23,32 +23,30 @@ int c0_of(int algo, const Scores &sc)
 }
 int b_of(int algo, const Scores &sc) { return algo == GLOBAL_ ? sc.mismatch - sc.e : sc.e; }
 
-cudaError_t pk_visit(int algo, int group, int start, bool fast, const PkLaunchFn &f)
+PkKernel pk_kernel(int algo, PkVariant v, int start)
 {
-    if (algo == LOCAL_) return pk_visit_local(group, start, fast, f);
-    if (algo == GLOBAL_) return pk_visit_global(group, start, fast, f);
-    return pk_visit_semi(group, start, fast, f);
+    if (algo == LOCAL_) return pk_kernel_local(v, start);
+    if (algo == GLOBAL_) return pk_kernel_global(v, start);
+    return pk_kernel_semi(v, start);
 }
 
 /* registers and static shared memory of a kernel, read once */
 struct KernelUse {
     int regs = 0, smem = 0;
 };
-KernelUse kernel_use(int algo, int group, int start, bool fast)
+KernelUse kernel_use(int algo, PkVariant v, int start)
 {
     static std::mutex mu;
-    static KernelUse cache[3][6][3][2];
+    static KernelUse cache[3][PK_VARIANTS][3];
     const int ai = algo == LOCAL_ ? 0 : algo == GLOBAL_ ? 1 : 2;
-    const int gi = group == 2 ? 0 : group == 4 ? 1 : group == 8 ? 2 : group == 16 ? 3 : 4;
     std::lock_guard<std::mutex> lk(mu);
-    KernelUse &u = cache[ai][gi][start][fast];
+    KernelUse &u = cache[ai][v][start];
     if (u.regs == 0) {
-        pk_visit(algo, group, start, fast, [&](PkKernel k) {
-            cudaFuncAttributes fa;
-            const cudaError_t e = cudaFuncGetAttributes(&fa, (const void *)k);
-            if (e == cudaSuccess) u.regs = fa.numRegs, u.smem = (int)fa.sharedSizeBytes;
-            return e;
-        });
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, (const void *)pk_kernel(algo, v, start)) == cudaSuccess)
+            u.regs = fa.numRegs, u.smem = (int)fa.sharedSizeBytes;
+        else
+            cudaGetLastError();
     }
     return u;
 }
@@ -109,75 +107,141 @@ PkConst pk_const(int algo, const Scores &sc)
     return p;
 }
 
-/* Lane group, block and grid of a launch over the pairs `sample` stands for.
- * A pair on G lanes takes rounds*words steps (rounds: its bands over 2G) and
- * as many more as the last round has bands, so narrow groups waste fewer lane-steps on fill, drain and the last
- * round, and wide ones give each pair less time and the chip more warps.  An
- * SM with A resident warps was modelled as running A/(A+4) of its peak rate
- * (a lone warp waits for its own dependency chains); the group with the least
- * modelled time is taken.  Rings (one word per query column and pair) bound
- * the resident warps of narrow groups on long queries. */
-WcLaunch pk_plan(int algo, int start, bool fast, int n, uint32_t max_q, const PkSample &sample, int sms, int forced)
+/* ring of a pair: a word per step of a round (an odd multiple of 4 words, so
+ * the 128-bit accesses of groups side by side hit different banks) */
+static int ring_words(int group, uint32_t max_q)
 {
-    WcLaunch best;
-    double best_t = 0;
-    for (int g : {2, 4, 8, 16, 32}) {
-        if (!fast && g != 8) continue;
-        if (fast && forced > 0 && g != forced) continue;
-        const KernelUse u = kernel_use(algo, g, start, fast);
-        const int V = 2 * g;
-        const size_t ring = std::max<size_t>((max_q + 7) & ~7u, 8 * V) * 4;
-        double steps = 0;
-        for (int k = 0; k < sample.n; k++) {
-            const int qw = sample.qw[k], nb = sample.tw[k];
-            const int rounds = (nb + V - 1) / V;
-            steps += (double)rounds * (rounds > 1 ? std::max(qw, V) : qw) + (nb + V - 1) % V;
-        }
-        steps /= std::max(sample.n, 1);
-        int res = 0, warps = 0;
-        for (int wpb : {2, 4, 1}) {
-            const int r = resident_warps(u, wpb, ring * wpb * (32 / g));
-            if (r > res) res = r, warps = wpb;
-        }
-        if (res == 0) continue;
-        const double total = ((double)n * g + 31) / 32 / sms; /* warps per SM */
-        const double t = total <= res ? steps * (total + 4) : steps * total * (res + 4) / res;
-        if (best.group == 0 || t < best_t) {
-            best_t = t;
-            if (total <= 4) warps = 1; /* small grids spread over the SMs */
-            best.group = g, best.warps = warps, best.smem = ring * warps * (32 / g);
-            best.resident_warps = res;
-            const int per_block = warps * 32 / g;
-            const int need = (n + per_block - 1) / per_block, cap = std::max(sms * res / warps, sms);
-            best.blocks = std::min(need, cap);
-        }
-    }
-    return best;
+    return std::max((int)((max_q + 7) & ~7u), 16 * group) + 4;
 }
 
-cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const uint32_t *list, int nlist,
-                         uint32_t max_q, const WcLaunch &fast, const WcLaunch &cmp, uint32_t *defer, uint32_t *wq,
-                         cudaStream_t s)
+/* steps of a pair of qw query words and nb bands on g lanes: rounds of its
+ * bands over 2g virtual lanes, and as many more as the last round has bands */
+static double steps_of(int g, int qw, int nb)
 {
-    if (nlist <= 0) return cudaSuccess;
-    auto launch = [&](const DpArgs &x, const uint32_t *l, const WcLaunch &w, bool is_fast) {
-        return pk_visit(algo, w.group, start, is_fast, [&](PkKernel k) {
-            const cudaError_t e = allow_dyn_smem_fn((const void *)k);
-            if (e != cudaSuccess) return e;
-            const int ring_cols = (int)std::max<uint32_t>((max_q + 7) & ~7u, 16u * w.group);
-            k<<<w.blocks, 32 * w.warps, w.smem, s>>>(x, pc, l, nlist, ring_cols);
-            return cudaGetLastError();
-        });
+    const int V = 2 * g, rounds = (nb + V - 1) / V;
+    return (double)rounds * (rounds > 1 ? std::max(qw, V) : qw) + (nb + V - 1) % V;
+}
+
+/* Lane group of each class, block and grid.  Narrow groups waste fewer
+ * lane-steps on fill, drain and the last round; wide ones give each pair less
+ * time and the chip more warps, and hold fewer rings.  A class's narrowest
+ * group is the one whose rings fit RING_WORDS per warp (14 of the 16 warps per
+ * SM that registers allow).  From there the longest pairs' groups are widened
+ * -- to 32 lanes, or to the block's two or four warps -- until the launch's
+ * modelled time, the larger of all warps' steps at the SMs' rate and any
+ * class's longest pair, stops falling.  A step of one of A resident warps of
+ * an SM is modelled as max(A, 4) + 2.5 units (one warp a scheduler waits for
+ * its own dependency chains: 65% of the integer pipe, two reach 73%); handing
+ * over between two or four warps costs 15 or 45% more (20 pairs of 250-2,000
+ * bp: 1,983 us with one warp, 1,427 with two, 1,236 with four). */
+bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPlan &p)
+{
+    constexpr int RING_WORDS = 4096 + 32 * 4;
+    constexpr int WIDE = 6; /* group index of the whole block; below: 1 << k lanes */
+    p = PkPlan();
+    uint32_t max_q = 0;
+    int n = 0;
+    for (int c = 0; c < PK_CLASSES; c++)
+        if (cl[c].n) n += cl[c].n, max_q = std::max(max_q, cl[c].max_q);
+    double best_t = 0;
+    for (int w : {1, 2, 4}) {
+        const KernelUse u = kernel_use(algo, w == 4 ? PK_W4 : w == 2 ? PK_W2 : PK_W1, start);
+        const double hand = w == 4 ? 1.45 : 1.15;
+        double cost[PK_CLASSES][WIDE + 1], longest[PK_CLASSES][WIDE + 1], limits[PK_CLASSES * (WIDE + 1)];
+        int low[PK_CLASSES], nlimits = 0;
+        const int top = w > 1 ? WIDE : WIDE - 1;
+        for (int c = 0; c < PK_CLASSES; c++) {
+            low[c] = 0;
+            if (cl[c].n == 0) continue;
+            const int qw = (int)((cl[c].max_q + 7) >> 3), tw = (int)((cl[c].max_t + 7) >> 3);
+            while (low[c] < WIDE - 1 && ring_words(1 << low[c], cl[c].max_q) * (32 >> low[c]) > RING_WORDS) low[c]++;
+            for (int k = low[c]; k <= top; k++) {
+                const int g = k == WIDE ? 32 * w : 1 << k;
+                const double f = k == WIDE ? hand : 1.0;
+                double steps = 0;
+                for (int x = 0; x < cl[c].ns; x++) steps += steps_of(g, cl[c].qw[x], cl[c].tw[x]);
+                cost[c][k] = f * steps / std::max(cl[c].ns, 1) * cl[c].n * g / 32;
+                longest[c][k] = f * steps_of(g, qw, tw);
+                limits[nlimits++] = longest[c][k];
+            }
+            while (low[c] < WIDE - 1 && cost[c][low[c] + 1] < cost[c][low[c]]) low[c]++;
+        }
+        for (int x = 0; x < nlimits; x++) {
+            int k[PK_CLASSES] = {}, words = 0;
+            size_t wide_words = 0;
+            double total = 0, work = 0, tail = 0;
+            for (int c = 0; c < PK_CLASSES; c++) {
+                if (cl[c].n == 0) continue;
+                k[c] = low[c];
+                if (forced > 32) k[c] = top;
+                else if (forced > 0) while (k[c] < WIDE - 1 && (1 << k[c]) < forced) k[c]++;
+                else while (k[c] < top && longest[c][k[c]] > limits[x]) k[c]++;
+                const int g = k[c] == WIDE ? 32 * w : 1 << k[c];
+                if (k[c] == WIDE)
+                    wide_words = std::max<size_t>(wide_words, ring_words(g, cl[c].max_q) + (w - 1) * 8 * PK_FIFO);
+                else words = std::max(words, ring_words(g, cl[c].max_q) * (32 / g));
+                total += (double)cl[c].n * g / 32;
+                work += cost[c][k[c]];
+                tail = std::max(tail, longest[c][k[c]]);
+            }
+            words = std::max(words, (int)((wide_words / w + 7) & ~3));
+            const int res = resident_warps(u, w, (size_t)words * w * 4);
+            if (res == 0) continue;
+            const double a = std::max(std::min(total / sms, (double)res), 1.0), step = std::max(a, 4.0) + 2.5;
+            const double t = std::max(work / sms / a, tail) * step;
+            if (p.warps == 0 || t < best_t) {
+                best_t = t;
+                p.warp_words = words, p.warps = w;
+                p.blocks = std::max(sms * res / w, sms);
+                for (int c = 0; c < PK_CLASSES; c++)
+                    if (cl[c].n) {
+                        p.group[c] = k[c] == WIDE ? 32 * w : 1 << k[c];
+                        p.ring_cols[c] = ring_words(p.group[c], cl[c].max_q);
+                    }
+            }
+        }
+    }
+    if (p.warps == 0) return false;
+    p.cmp_cols = ring_words(8, max_q);
+    const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1, (size_t)p.cmp_cols * 16);
+    p.cmp_blocks = std::min((n + 3) / 4, std::max(sms * res, sms));
+    return res > 0;
+}
+
+cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const PkPlan &p, const uint32_t *list,
+                         const int *n, uint32_t *defer, uint32_t *wq, cudaStream_t s)
+{
+    PkClasses cl;
+    int total = 0;
+    long warps = 0;
+    cl.warp_words = p.warp_words;
+    for (int c = 0; c < PK_CLASSES; c++) {
+        if (n[c] == 0) continue;
+        cl.k[cl.n++] = {p.group[c], total, n[c], p.ring_cols[c]};
+        warps += ((long)n[c] * p.group[c] + 31) / 32;
+        total += n[c];
+    }
+    if (total == 0) return cudaSuccess;
+    auto launch = [&](PkVariant which, const DpArgs &x, const PkClasses &k, const uint32_t *l, int nb, int w) {
+        const PkKernel f = pk_kernel(algo, which, start);
+        const cudaError_t e = allow_dyn_smem_fn((const void *)f);
+        if (e != cudaSuccess) return e;
+        f<<<nb, 32 * w, (size_t)k.warp_words * w * 4, s>>>(x, pc, k, l);
+        return cudaGetLastError();
     };
     /* the table-scoring launch, then the compare-scoring one over the pairs it
      * left (a target with another code than A, C, G, T, N) */
     DpArgs f = a;
-    f.queue = wq, f.defer = defer, f.ndefer = wq + 2, f.n_dev = nullptr;
-    cudaError_t e = launch(f, list, fast, true);
+    f.queue = wq, f.defer = defer, f.ndefer = wq + PK_CLASSES + 1, f.n_dev = nullptr, f.stuck = wq + PK_CLASSES + 2;
+    cudaError_t e = launch(p.warps == 4 ? PK_W4 : p.warps == 2 ? PK_W2 : PK_W1, f, cl, list,
+                           (int)std::min<long>((warps + p.warps - 1) / p.warps, p.blocks), p.warps);
     if (e != cudaSuccess) return e;
-    DpArgs c = a;
-    c.queue = wq + 1, c.defer = nullptr, c.ndefer = nullptr, c.n_dev = wq + 2;
-    return launch(c, defer, cmp, false);
+    DpArgs c = f;
+    c.queue = wq + PK_CLASSES, c.defer = nullptr, c.ndefer = nullptr, c.n_dev = f.ndefer;
+    PkClasses one;
+    one.n = 1, one.warp_words = 4 * p.cmp_cols;
+    one.k[0] = {8, 0, total, p.cmp_cols};
+    return launch(PK_CMP, c, one, defer, std::min((total + 3) / 4, p.cmp_blocks), 1);
 }
 
 } // namespace gb

@@ -31,6 +31,15 @@
  * cell and the shuffles, and keeps one ring per pair (packing two pairs per
  * lane instead doubles the rings and halves the resident warps).
  *
+ * W = 2 and 4: the warps of a block share a pair, for pairs that would outlast
+ * the rest of the launch.  Warp x takes the bands of every W-th round; the warps run
+ * unsynchronised, each
+ * handing its last virtual lane's outputs to the next through a fifo of
+ * PK_FIFO words with counters (bounded waits), the last to the first through
+ * the ring.  No warp waits in a circle: a round has at least as many steps as
+ * the group virtual lanes, and the ring holds a whole one, so the last warp
+ * never waits for room.
+ *
  * H and E cross a band boundary as 16-bit values, as in the reference's short2
  * row buffer; the host only sends pairs here whose values cannot leave 15 bits
  * (pk_fits), so the results are the reference's bit for bit.
@@ -47,9 +56,7 @@ namespace gb {
 namespace {
 
 constexpr uint32_t PAD_WORD = 0xEEEEEEEEu; /* eight N codes */
-#ifndef PK_MIN_BLOCKS
-#define PK_MIN_BLOCKS 4
-#endif
+constexpr int PK_SPINS = 1 << 22;          /* bound of a wait on another warp of the group */
 
 __device__ __forceinline__ int half_of(uint32_t x, bool hi) { return (int)(int16_t)(hi ? x >> 16 : x & 0xFFFFu); }
 /* both halves of x with half `hi` replaced by v (16 bits) */
@@ -98,34 +105,49 @@ __device__ void pk_score_table(uint2 *tab, const Scores &sc, bool n_zero, int ab
     for (int x = threadIdx.x; x < 256; x += blockDim.x) tab[x] = make_uint2(row(x >> 4), row(x & 15));
 }
 
-/* FAST: targets of A, C, G, T and N, scores by one prmt per packed cell (its
+/* The pairs list[0..nl) on G lanes of W warps each, taken from the zeroed
+ * counter `queue`.  smem: the warp's rings (W > 1: the block's).
+ * FAST: targets of A, C, G, T and N, scores by one prmt per packed cell (its
  * selector's bytes: the row's class, then that byte's sign).  Otherwise
  * compares, any code. */
-template <int G, int ALGO, int START, bool FAST>
-__global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_constant__ DpArgs A, const __grid_constant__ PkConst P,
-                                                    const uint32_t *list, int nlist, int ring_cols)
+template <int G, int W, int ALGO, int START, bool FAST>
+__device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, const uint2 *tab, uint32_t *pk_smem,
+                                         const uint32_t *list, int nl, uint32_t *queue, int ring_cols)
 {
+    constexpr int LANES = G * W;
     constexpr int V = 2 * G;
     constexpr bool LOC = ALGO == LOCAL_, GLO = ALGO == GLOBAL_, SEM = ALGO == SEMI_GLOBAL_;
     constexpr bool TB = START == WITH_TB_;
-    extern __shared__ __align__(16) uint32_t pk_smem[];
-    __shared__ uint2 tab[FAST ? 256 : 1];
-    if (FAST) {
-        pk_score_table(tab, A.sc, !GLO, P.a + P.b);
-        __syncthreads();
-    }
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), gbase = lane & ~(G - 1);
     const unsigned gmask = G == 32 ? 0xFFFFFFFFu : (((1u << (G & 31)) - 1u) << gbase);
-    uint32_t *ring = pk_smem + (size_t)(threadIdx.x / G) * ring_cols;
-    const int nl = A.n_dev ? min((int)*A.n_dev, nlist) : nlist;
     const int o = A.sc.o, e = A.sc.e, oe = A.sc.oe;
     const bool free_head_t = SEM && (A.head == TARGET_ || A.head == BOTH_);
     const bool zero_rows = SEM && (A.head == QUERY_ || A.head == BOTH_);
+    const int wi = W > 1 ? (int)(threadIdx.x >> 5) : 0;
+    /* the last warp's outputs to the first: a word per query column; between
+     * neighbouring warps of a group: PK_FIFO query words */
+    uint32_t *ring = pk_smem + (W > 1 ? 0 : (size_t)(lane / G) * ring_cols);
+    uint32_t *fifo = pk_smem + ring_cols; /* warp w's at fifo + w * 8 * PK_FIFO */
+    /* W > 1: query words handed on and taken, counted over the rounds; a start
+     * pass's first band with a hit; the group's item and results */
+    __shared__ volatile int prod[W], cons[W], s_stop;
+    __shared__ int s_item, s_key[W], s_res[3];
+    auto group_any = [&](bool x) -> bool {
+        if (W > 1) return __syncthreads_or(x);
+        return __ballot_sync(0xFFFFFFFFu, x) & gmask;
+    };
 
     for (;;) {
         unsigned item0 = 0;
-        if (lane == 0) item0 = atomicAdd(A.queue, (unsigned)(32 / G));
-        item0 = __shfl_sync(0xFFFFFFFFu, item0, 0);
+        if (W > 1) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
+            __syncthreads();
+            item0 = (unsigned)s_item;
+        } else {
+            if (lane == 0) item0 = atomicAdd(queue, (unsigned)(32 / G));
+            item0 = __shfl_sync(0xFFFFFFFFu, item0, 0);
+        }
         if ((int)item0 >= nl) break;
         const int item = (int)item0 + lane / G;
         const bool listed = item < nl;
@@ -136,19 +158,20 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
         bool has = listed, with_n = false;
         if (FAST) {
             uint32_t odd = 0, odd_q = 0;
-            for (int x = gl; 8 * x < tlen0; x += G) odd |= odd_codes(t[x], tlen0 - 8 * x);
+            const int x0 = W > 1 ? (int)threadIdx.x : gl;
+            for (int x = x0; 8 * x < tlen0; x += LANES) odd |= odd_codes(t[x], tlen0 - 8 * x);
             bool bad = odd & 1u;
             if (GLO) {
                 /* N is an ordinary base: a target N scores as against A, C, G or T unless the
                  * query has N too (with a traceback, either one's N meets the other's pads) */
-                for (int x = gl; 8 * x < qlen0; x += G) odd_q |= odd_codes(q[x], qlen0 - 8 * x);
-                const bool tn = __ballot_sync(0xFFFFFFFFu, odd & 2u) & gmask;
+                for (int x = x0; 8 * x < qlen0; x += LANES) odd_q |= odd_codes(q[x], qlen0 - 8 * x);
+                const bool tn = group_any(odd & 2u);
                 bad |= TB ? tn || (odd_q & 2u) : tn && (odd_q & 2u);
             } else {
-                with_n = __any_sync(0xFFFFFFFFu, odd & 6u);
+                with_n = W > 1 ? group_any(odd & 6u) : __any_sync(0xFFFFFFFFu, odd & 6u);
             }
-            if (__ballot_sync(0xFFFFFFFFu, bad) & gmask) {
-                if (listed && gl == 0) A.defer[atomicAdd(A.ndefer, 1u)] = (uint32_t)i;
+            if (group_any(bad)) {
+                if (listed && gl == 0 && wi == 0) A.defer[atomicAdd(A.ndefer, 1u)] = (uint32_t)i;
                 has = false;
             }
         }
@@ -160,7 +183,7 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
             tops = reinterpret_cast<uint32_t *>(A.tb + A.tb_off[i]);
             lefts = tops + (size_t)((tregs + 1) >> 1) * (qregs << 3);
         }
-        if (TB && has && gl == 0) A.tb_kind[i] = 1;
+        if (TB && has && gl == 0 && wi == 0) A.tb_kind[i] = 1;
         int score = 0, r_qe = 0, r_te = 0, r_qs = 0, r_ts = 0;
 
 #pragma unroll 1
@@ -177,11 +200,25 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                 T0 = max(x > 0 ? x - 1 : x, 0);
                 nb = work ? tregs - T0 : 0;
             }
-            const int rounds = qn > 0 ? (nb + V - 1) / V : 0;
-            const int per = rounds > 1 ? max(qn, V) : qn; /* steps of a round: the ring's reader trails its writer */
-            int gend = rounds > 0 ? rounds * per + ((nb - 1) & (V - 1)) : 0; /* the last band's virtual lane is done */
-            int wend = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)gend);
-            const bool multi = wend > 0 && __any_sync(0xFFFFFFFFu, rounds > 1);
+            /* rounds of warp x of the group: it takes bands (r*W + x)*V .. of round r */
+            auto rounds_of = [&](int x) { return qn > 0 && nb > x * V ? (nb - x * V + W * V - 1) / (W * V) : 0; };
+            const int rounds = rounds_of(wi);
+            /* steps of a round: the group's first virtual lane comes to a word of the next
+             * round after the last one has done it */
+            const int per = rounds_of(0) > 1 ? max(qn, W * V) : qn;
+            /* done when the last band's virtual lane is */
+            int gend = rounds > 0 ? rounds * per + min(V - 1, nb - 1 - ((rounds - 1) * W + wi) * V) : 0;
+            int wend = W > 1 ? gend : (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)gend);
+            const bool multi = W == 1 && wend > 0 && __any_sync(0xFFFFFFFFu, rounds > 1);
+            /* words the next warp will take from this one, and where */
+            const int wanted = W == 1 ? 0 : wi < W - 1 ? rounds_of(wi + 1) * per : (rounds_of(0) - 1) * per;
+            int avail = 0, taken = 0;
+            if (W > 1) {
+                __syncthreads();
+                if (lane == 0) prod[wi] = 0, cons[wi] = 0;
+                if (threadIdx.x == 0) s_stop = 0x7fffffff, s_res[0] = s_res[1] = s_res[2] = 0;
+                __syncthreads();
+            }
             const int lastw = (qlen - 1) >> 3, lastb = (qlen - 1) & 7;
 
             auto qword = [&](int j) -> uint32_t {
@@ -212,7 +249,9 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                 sel[k] = 0;
             }
             int w = -2 * gl, r = 0, wh = w - 1, rh = 0;
-            uint32_t qw = qword(w), qp = PAD_WORD, qx = qword(w + 1);
+            uint32_t qw = qword(w), qp = PAD_WORD;
+            /* the halves' next bands' words, loaded a round ahead of use */
+            uint32_t t_lo = tword(wi * V + 2 * gl), t_hi = tword(wi * V + 2 * gl + 1);
             /* LOCAL: key of the best cell so far (4 * H + 3), per half; a start
              * pass looks for the forward score.  SEMI_GLOBAL: best last-column
              * value, in basis (0, lastb) */
@@ -231,7 +270,25 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
 #pragma unroll
             for (int k = 0; k < 8; k++) nrow[k] = 0;
             for (int s = 0; s < wend; s++) {
-                const int band_lo = r * V + 2 * gl, band_hi = rh * V + 2 * gl + 1;
+                const int band_lo = (r * W + wi) * V + 2 * gl, band_hi = (rh * W + wi) * V + 2 * gl + 1;
+                if (W > 1 && s < rounds * per) { /* wait for the word that lane 0 reads */
+                    const int src = wi > 0 ? wi - 1 : W - 1, need = wi > 0 ? s : s - per;
+                    for (int spin = 0; need >= avail;) {
+                        avail = prod[src];
+                        if (need < 0) break;
+                        if (++spin > PK_SPINS) {
+                            *A.stuck = 1u; /* never: the producer's step does not wait on this one */
+                            wend = s;
+                            break;
+                        }
+                    }
+                    __syncwarp();
+                    __threadfence_block();
+                }
+                /* next step's query word: in flight during this one (and before the fence that
+                 * ends it, which waits for loads) */
+                const uint32_t qx = qword(w + 1 == per ? 0 : w + 1);
+                const int stop_seen = W > 1 && rev ? s_stop : 0x7fffffff;
                 const bool on = s < gend;
                 const bool live_lo = on && w >= 0 && band_lo < nb, live_hi = on && wh >= 0 && band_hi < nb;
                 /* H and E entering the low half's band at this word's columns */
@@ -239,7 +296,7 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
 #pragma unroll
                 for (int b = 0; b < 8; b++) xin[b] = __shfl_up_sync(0xFFFFFFFFu, xw[b], 1, G);
                 if (gl == 0) {
-                    if (r == 0 || r >= rounds) { /* past the last round: values no carry can come from */
+                    if ((r == 0 && wi == 0) || r >= rounds) { /* past the last round: values no carry can come from */
 #pragma unroll
                         for (int b = 0; b < 8; b++) {
                             const int c = (w << 3) + b;
@@ -252,11 +309,16 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                             xin[b] = (uint32_t)hb | ((uint32_t)eb << 16);
                         }
                     } else {
-                        const uint4 *rp = reinterpret_cast<const uint4 *>(ring + (w << 3));
+                        const uint4 *rp = reinterpret_cast<const uint4 *>(
+                            W > 1 && wi > 0 ? fifo + ((wi - 1) * PK_FIFO + (s & (PK_FIFO - 1))) * 8 : ring + (w << 3));
                         const uint4 x0 = rp[0], x1 = rp[1];
                         xin[0] = x0.x, xin[1] = x0.y, xin[2] = x0.z, xin[3] = x0.w;
                         xin[4] = x1.x, xin[5] = x1.y, xin[6] = x1.z, xin[7] = x1.w;
                     }
+                }
+                if (W > 1 && wi > 0 && lane == 0) {
+                    __threadfence_block();
+                    cons[wi] = s + 1;
                 }
                 if (TB && live_lo && w < qregs) {
                     uint4 *p4 = reinterpret_cast<uint4 *>(tops + (size_t)(band_lo >> 1) * (qregs << 3) + (w << 3));
@@ -268,7 +330,9 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                 for (int h = 0; h < 2; h++) {
                     if ((h ? wh : w) == 0) {
                         const int band = h ? band_hi : band_lo;
-                        const uint32_t tw = tword(band);
+                        const uint32_t tw = h ? t_hi : t_lo;
+                        if (h) t_hi = tword(band + W * V);
+                        else t_lo = tword(band + W * V);
                         const int R0 = band < nb ? band << 3 : 0;
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
@@ -393,6 +457,30 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                     }
                     __syncwarp();
                 }
+                if (W > 1) {
+                    const int x = s - (V - 1); /* the word the last virtual lane has done */
+                    if (x >= 0 && x < wanted && on) {
+                        if (wi < W - 1) {
+                            for (int spin = 0; taken + PK_FIFO <= x;) { /* room in the fifo */
+                                taken = cons[wi + 1];
+                                if (++spin > PK_SPINS) {
+                                    *A.stuck = 1u;
+                                    wend = s;
+                                    break;
+                                }
+                            }
+                            __syncwarp();
+                        }
+                        if (gl == G - 1) {
+                            uint4 *rp = reinterpret_cast<uint4 *>(
+                                wi < W - 1 ? fifo + (wi * PK_FIFO + (x & (PK_FIFO - 1))) * 8 : ring + (wh << 3));
+                            rp[0] = make_uint4(xw[0], xw[1], xw[2], xw[3]);
+                            rp[1] = make_uint4(xw[4], xw[5], xw[6], xw[7]);
+                            __threadfence_block();
+                            prod[wi] = x + 1;
+                        }
+                    }
+                }
                 bool hit = false;
                 if (LOC) {
                     const uint32_t m = __vmaxs2(bk, thr);
@@ -466,34 +554,54 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                                 if (hit_lo) bd = min(bd, (at_lo >> 3) - T0);
                                 if (hit_hi) bd = min(bd, (at_hi >> 3) - T0);
                             }
-                            if (bd != 0x7fffffff) fin = (bd / V) * per + per + (bd % V);
+                            if (W > 1) atomicMin(const_cast<int *>(&s_stop), bd);
+                            else if (bd != 0x7fffffff) fin = (bd / V) * per + per + (bd % V);
                         }
+                        if (W == 1) {
 #pragma unroll
-                        for (int off = G / 2; off > 0; off >>= 1)
-                            fin = min(fin, __shfl_xor_sync(0xFFFFFFFFu, fin, off));
+                            for (int off = G / 2; off > 0; off >>= 1)
+                                fin = min(fin, __shfl_xor_sync(0xFFFFFFFFu, fin, off));
+                            gend = min(gend, max(fin, s + 1));
+                            wend = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)gend);
+                        }
+                    }
+                    if (W > 1 && __any_sync(0xFFFFFFFFu, stop_seen != 0x7fffffff)) {
+                        const int bd = (int)__reduce_min_sync(0xFFFFFFFFu, (unsigned)stop_seen);
+                        const int R = bd / (W * V), wb = bd / V - R * W, vb = bd % V;
+                        int fin = R * per + V; /* the rounds before */
+                        if (wi < wb) fin += per;
+                        else if (wi == wb) fin = max(fin, R * per + per + vb);
                         gend = min(gend, max(fin, s + 1));
-                        wend = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)gend);
+                        wend = min(wend, gend);
                     }
                 }
                 wh = w, rh = r;
                 if (++w == per) w = 0, ++r;
                 qp = qw, qw = qx;
-                const int wn = w + 1 == per ? 0 : w + 1;
-                qx = qword(wn);
             }
             };
             if (FAST && !GLO && with_n) sweep(std::true_type{});
             else sweep(std::false_type{});
+            if (W > 1) { /* nobody waits for a warp that is done */
+                __syncwarp();
+                if (lane == 0) prod[wi] = 0x3fffffff, cons[wi] = 0x3fffffff;
+            }
 
             /* the pair's result from its virtual lanes */
             if (GLO) {
-                const unsigned own = __ballot_sync(0xFFFFFFFFu, at_lo == 1) & gmask;
-                score = __shfl_sync(0xFFFFFFFFu, score, own ? __ffs((int)own) - 1 : lane);
-                if (!own) score = 0;
+                if (W > 1) {
+                    if (at_lo == 1) s_res[0] = score;
+                    __syncthreads();
+                    score = s_res[0];
+                } else {
+                    const unsigned own = __ballot_sync(0xFFFFFFFFu, at_lo == 1) & gmask;
+                    score = __shfl_sync(0xFFFFFFFFu, score, own ? __ffs((int)own) - 1 : lane);
+                    if (!own) score = 0;
+                }
             } else {
                 unsigned best = 0;
                 bool use_hi = false;
-                const bool any_hit = SEM && rev && (__ballot_sync(0xFFFFFFFFu, hit_lo || hit_hi) & gmask);
+                const bool any_hit = SEM && rev && group_any(hit_lo || hit_hi);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int at = h ? at_hi : at_lo;
@@ -513,9 +621,15 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                 unsigned all = best;
 #pragma unroll
                 for (int off = G / 2; off > 0; off >>= 1) all = max(all, __shfl_xor_sync(0xFFFFFFFFu, all, off));
+                if (W > 1) {
+                    if (lane == 0) s_key[wi] = (int)all;
+                    __syncthreads();
+#pragma unroll
+                    for (int x = 0; x < W; x++) all = max(all, (unsigned)s_key[x]);
+                }
                 const bool mine = all != 0 && best == all;
-                const unsigned own = __ballot_sync(0xFFFFFFFFu, mine) & gmask;
-                const int src = own ? __ffs((int)own) - 1 : lane;
+                const unsigned own = W > 1 ? all : __ballot_sync(0xFFFFFFFFu, mine) & gmask;
+                const int src = W == 1 && own ? __ffs((int)own) - 1 : lane;
                 int row = 0, col = 0, val = 0;
                 if (LOC && mine) {
                     /* the block's first column reaching the value, its first row */
@@ -533,9 +647,15 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
                     row = (band << 3) + kr, col = (word << 3) + bb;
                 }
                 if (SEM && mine) row = use_hi ? at_hi : at_lo, val = half_of(thr, use_hi) - sbase;
-                row = __shfl_sync(0xFFFFFFFFu, row, src);
-                col = __shfl_sync(0xFFFFFFFFu, col, src);
-                val = __shfl_sync(0xFFFFFFFFu, val, src);
+                if (W > 1) {
+                    if (mine) s_res[0] = row, s_res[1] = col, s_res[2] = val;
+                    __syncthreads();
+                    row = s_res[0], col = s_res[1], val = s_res[2];
+                } else {
+                    row = __shfl_sync(0xFFFFFFFFu, row, src);
+                    col = __shfl_sync(0xFFFFFFFFu, col, src);
+                    val = __shfl_sync(0xFFFFFFFFu, val, src);
+                }
                 if (!rev) {
                     score = val, r_te = row, r_qe = LOC ? col : tlen;
                 } else if (LOC) {
@@ -547,7 +667,7 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
             }
         }
 
-        if (gl == 0 && has) {
+        if (gl == 0 && wi == 0 && has) {
             if (A.score) A.score[i] = score;
             if (!GLO) {
                 if (A.q_end) A.q_end[i] = r_qe;
@@ -561,30 +681,63 @@ __global__ void __launch_bounds__(128, PK_MIN_BLOCKS) dp_pk_kernel(const __grid_
     }
 }
 
-template <int ALGO, bool FAST, class F> cudaError_t pk_with_group(int group, int start, F &&f)
+/* One launch over every class of pairs, longest first: a warp works through
+ * the first class's pairs with that class's lane group, then the next's, so no
+ * class has a tail of its own and a batch of mixed lengths fills the chip to
+ * its end (launches per class, one after another or on two streams, left
+ * 10,000 pairs of 50-1,000 bp at 3.1 ms).  A class of group 32 * W shares each
+ * pair among the W warps of the block. */
+template <int W, int ALGO, int START, bool FAST>
+__global__ void __launch_bounds__(32 * W, 16 / W)
+    dp_pk_kernel(const __grid_constant__ DpArgs A, const __grid_constant__ PkConst P,
+                 const __grid_constant__ PkClasses C, const uint32_t *list)
 {
-#define GB_PK_START(G)                                                                         \
-    do {                                                                                       \
-        if (start == WITH_TB_ && ALGO != SEMI_GLOBAL_)                                         \
-            return f(dp_pk_kernel<G, ALGO, ALGO == SEMI_GLOBAL_ ? WITHOUT_START_ : WITH_TB_, FAST>); \
-        if (start == WITH_START_ && ALGO != GLOBAL_)                                           \
-            return f(dp_pk_kernel<G, ALGO, ALGO == GLOBAL_ ? WITHOUT_START_ : WITH_START_, FAST>);   \
-        return f(dp_pk_kernel<G, ALGO, WITHOUT_START_, FAST>);                                 \
-    } while (0)
-    if constexpr (FAST) {
-        if (group == 2) GB_PK_START(2);
-        if (group == 4) GB_PK_START(4);
-        if (group == 16) GB_PK_START(16);
-        if (group == 32) GB_PK_START(32);
+    extern __shared__ __align__(16) uint32_t pk_smem[];
+    __shared__ uint2 tab[FAST ? 256 : 1];
+    if (FAST) {
+        pk_score_table(tab, A.sc, ALGO != GLOBAL_, P.a + P.b);
+        __syncthreads();
     }
-    if (group == 8) GB_PK_START(8);
-#undef GB_PK_START
-    return cudaErrorInvalidValue;
+    uint32_t *mem = pk_smem + (size_t)(threadIdx.x >> 5) * C.warp_words;
+#pragma unroll 1
+    for (int c = 0; c < C.n; c++) {
+        const PkClass &k = C.k[c];
+        const uint32_t *l = list ? list + k.first : nullptr;
+        const int nl = A.n_dev ? min((int)*A.n_dev, k.n) : k.n;
+        uint32_t *qu = A.queue + c;
+        if (!FAST) {
+            pk_pairs<8, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols);
+            continue;
+        }
+        switch (k.group) {
+        case 1: pk_pairs<1, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 2: pk_pairs<2, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 4: pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 8: pk_pairs<8, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 16: pk_pairs<16, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 32: pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        default:
+            if constexpr (W > 1) pk_pairs<32, W, ALGO, START, FAST>(A, P, tab, pk_smem, l, nl, qu, k.ring_cols);
+            __syncthreads(); /* the block's rings become its warps' */
+        }
+    }
 }
 
-template <int ALGO> cudaError_t pk_visit(int group, int start, bool fast, const PkLaunchFn &f)
+template <int ALGO, int START> PkKernel pk_variant(PkVariant v)
 {
-    return fast ? pk_with_group<ALGO, true>(group, start, f) : pk_with_group<ALGO, false>(group, start, f);
+    if (v == PK_CMP) return dp_pk_kernel<1, ALGO, START, false>;
+    if (v == PK_W4) return dp_pk_kernel<4, ALGO, START, true>;
+    if (v == PK_W2) return dp_pk_kernel<2, ALGO, START, true>;
+    return dp_pk_kernel<1, ALGO, START, true>;
+}
+
+template <int ALGO> PkKernel pk_kernel(PkVariant v, int start)
+{
+    if (start == WITH_TB_ && ALGO != SEMI_GLOBAL_)
+        return pk_variant<ALGO, ALGO == SEMI_GLOBAL_ ? WITHOUT_START_ : WITH_TB_>(v);
+    if (start == WITH_START_ && ALGO != GLOBAL_)
+        return pk_variant<ALGO, ALGO == GLOBAL_ ? WITHOUT_START_ : WITH_START_>(v);
+    return pk_variant<ALGO, WITHOUT_START_>(v);
 }
 
 } // namespace

@@ -29,18 +29,41 @@ struct PkConst {
     uint32_t kc[8];     /* LOCAL: packed -4*b*(bc+1) */
 };
 
-using PkKernel = void (*)(DpArgs, PkConst, const uint32_t *, int, int);
-using PkLaunchFn = std::function<cudaError_t(PkKernel)>;
+/* query words between neighbouring warps of a multi-warp group */
+constexpr int PK_FIFO = 32;
 
-/* calls f with the kernel of (algo, group, start, scoring) */
-cudaError_t pk_visit_local(int group, int start, bool fast, const PkLaunchFn &f);
-cudaError_t pk_visit_global(int group, int start, bool fast, const PkLaunchFn &f);
-cudaError_t pk_visit_semi(int group, int start, bool fast, const PkLaunchFn &f);
+/* One class of a launch: pairs list[first, first + n) on `group` lanes each
+ * (32 * the block's warps: the block), with rings of ring_cols words. */
+struct PkClass {
+    int32_t group, first, n, ring_cols;
+};
+constexpr int PK_CLASSES = 6;
+struct PkClasses {
+    int32_t n = 0, warp_words = 0; /* shared memory of a warp */
+    PkClass k[PK_CLASSES] = {};
+};
 
-/* lengths (words) of up to 256 pairs standing for a launch's */
-struct PkSample {
+using PkKernel = void (*)(DpArgs, PkConst, PkClasses, const uint32_t *);
+/* compare scoring (8 lanes to a pair); table scoring in blocks of 1, 2, 4 warps */
+enum PkVariant { PK_CMP, PK_W1, PK_W2, PK_W4, PK_VARIANTS };
+PkKernel pk_kernel_local(PkVariant v, int start);
+PkKernel pk_kernel_global(PkVariant v, int start);
+PkKernel pk_kernel_semi(PkVariant v, int start);
+
+/* lengths of the pairs of one class: their number, the longest, and (words)
+ * up to 128 of them */
+struct PkLengths {
     int n = 0;
-    int qw[256], tw[256];
+    uint32_t max_q = 0, max_t = 0, max_min = 0;
+    int ns = 0;
+    int qw[128], tw[128];
+};
+/* the shapes of a batch's launches */
+struct PkPlan {
+    int group[PK_CLASSES] = {};
+    int ring_cols[PK_CLASSES] = {};
+    int warp_words = 0, warps = 0, blocks = 0;         /* blocks: most that are resident */
+    int cmp_cols = 0, cmp_blocks = 0;
 };
 
 /* The packed kernels take LOCAL, GLOBAL and target-tail SEMI_GLOBAL without a
@@ -50,13 +73,13 @@ struct PkSample {
 bool pk_scores_ok(int algo, const Scores &sc);
 bool pk_fits(int algo, const Scores &sc, uint32_t max_q, uint32_t max_t, uint32_t max_min);
 PkConst pk_const(int algo, const Scores &sc);
-/* launch shape for n pairs (forced: a lane group, 0 = by the model) */
-WcLaunch pk_plan(int algo, int start, bool fast, int n, uint32_t max_q, const PkSample &sample, int sms, int forced);
-/* wq: three zeroed words (the two launches' work counters, the count of
- * pairs the first leaves to the second); defer: nlist words */
-cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const uint32_t *list, int nlist,
-                         uint32_t max_q, const WcLaunch &fast, const WcLaunch &cmp, uint32_t *defer, uint32_t *wq,
-                         cudaStream_t s);
+/* false: no shape fits.  forced: lanes per pair (8, 16, 32, 64), 0 = by the model */
+bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPlan &p);
+/* n[c]: the pairs of class c, in list order.  wq: PK_QUEUE_WORDS zeroed words;
+ * defer: a word per pair */
+constexpr int PK_QUEUE_WORDS = PK_CLASSES + 3;
+cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const PkPlan &p, const uint32_t *list,
+                         const int *n, uint32_t *defer, uint32_t *wq, cudaStream_t s);
 
 } // namespace gb
 

@@ -2,8 +2,5 @@
 #include "dp_pk.cuh"
 
 namespace gb {
-cudaError_t pk_visit_global(int group, int start, bool fast, const PkLaunchFn &f)
-{
-    return pk_visit<GLOBAL_>(group, start, fast, f);
-}
+PkKernel pk_kernel_global(PkVariant v, int start) { return pk_kernel<GLOBAL_>(v, start); }
 } // namespace gb

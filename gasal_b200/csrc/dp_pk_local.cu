@@ -2,8 +2,5 @@
 #include "dp_pk.cuh"
 
 namespace gb {
-cudaError_t pk_visit_local(int group, int start, bool fast, const PkLaunchFn &f)
-{
-    return pk_visit<LOCAL_>(group, start, fast, f);
-}
+PkKernel pk_kernel_local(PkVariant v, int start) { return pk_kernel<LOCAL_>(v, start); }
 } // namespace gb

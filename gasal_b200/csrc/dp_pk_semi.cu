@@ -2,8 +2,5 @@
 #include "dp_pk.cuh"
 
 namespace gb {
-cudaError_t pk_visit_semi(int group, int start, bool fast, const PkLaunchFn &f)
-{
-    return pk_visit<SEMI_GLOBAL_>(group, start, fast, f);
-}
+PkKernel pk_kernel_semi(PkVariant v, int start) { return pk_kernel<SEMI_GLOBAL_>(v, start); }
 } // namespace gb

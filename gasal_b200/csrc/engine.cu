@@ -236,10 +236,11 @@ static int ensure_order_buffers(Workspace &ws, size_t n)
     return GB_OK;
 }
 
-static int pk_class_of(uint32_t qlen)
+static int pk_class_of(uint32_t qlen, uint32_t tlen)
 {
     const uint32_t words = (qlen + 7) >> 3;
-    int c = 0;
+    if (words >= ORDER_CAP_WORDS) return order_prefix_units(words, (tlen + 7) >> 3) >= PK_LONG_UNITS ? 0 : 1;
+    int c = 2;
     while (words < PK_CLASS_WORDS[c]) c++;
     return c;
 }
@@ -258,64 +259,55 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
                          (cfg.algo == SEMI_GLOBAL_ && cfg.tail == TARGET_ && cfg.start != WITH_TB_);
     if (!algo_ok || !st.persistent || (cfg.second && cfg.algo != GLOBAL_) || !pk_scores_ok(cfg.algo, cfg.sc))
         return GB_OK;
-    struct {
-        int n = 0;
-        uint32_t max_q = 0, max_t = 0, max_min = 0;
-        PkSample sample;
-    } cl[PK_CLASSES];
+    PkLengths cl[PK_CLASSES];
     uint32_t min_q = 0xFFFFFFFFu, max_q = 0;
-    const int stride = std::max(1, b.n / 1024);
+    const int stride = std::max(1, b.n / 512);
     for (int i = 0, next = 0; i < b.n; i++) {
         const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
-        auto &c = cl[pk_class_of(ql)];
+        PkLengths &c = cl[pk_class_of(ql, tl)];
         c.n++;
         c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl), c.max_min = std::max(c.max_min, std::min(ql, tl));
         min_q = std::min(min_q, ql), max_q = std::max(max_q, ql);
-        if (i == next) {
+        if (i >= next && c.ns < 128) {
             next += stride;
-            PkSample &sm = c.sample;
-            if (sm.n < 256) sm.qw[sm.n] = (int)((ql + 7) >> 3), sm.tw[sm.n] = (int)((tl + 7) >> 3), sm.n++;
+            c.qw[c.ns] = (int)((ql + 7) >> 3), c.tw[c.ns] = (int)((tl + 7) >> 3), c.ns++;
         }
     }
     /* an unordered batch is one class: equal lengths, or too few pairs for the order to matter */
     const bool order = b.n >= st.min_order_pairs || (b.n > 64 && st.min_order_pairs <= (1 << 29) && max_q > min_q + min_q / 2);
     if (!order) {
-        auto &z = cl[0];
+        PkLengths &z = cl[0];
         for (int c = 1; c < PK_CLASSES; c++) {
             z.n += cl[c].n;
             z.max_q = std::max(z.max_q, cl[c].max_q), z.max_t = std::max(z.max_t, cl[c].max_t);
             z.max_min = std::max(z.max_min, cl[c].max_min);
-            for (int k = 0; k < cl[c].sample.n && z.sample.n < 256; k++, z.sample.n++)
-                z.sample.qw[z.sample.n] = cl[c].sample.qw[k], z.sample.tw[z.sample.n] = cl[c].sample.tw[k];
-            cl[c].n = 0;
+            for (int k = 0; k < cl[c].ns && z.ns < 128; k++, z.ns++) z.qw[z.ns] = cl[c].qw[k], z.tw[z.ns] = cl[c].tw[k];
+            cl[c].n = cl[c].ns = 0;
         }
     }
     p.pk_wc = false;
     for (int c = 0; c < PK_CLASSES; c++) {
         if (cl[c].n == 0) continue;
         if (!pk_fits(cfg.algo, cfg.sc, cl[c].max_q, cl[c].max_t, cl[c].max_min)) {
-            if (c > 0 || !order) return GB_OK;
+            if (c > 1 || !order) return GB_OK;
             p.pk_wc = true;
+            cl[0].n = cl[1].n = 0;
             continue;
         }
-        if (cl[c].sample.n == 0) {
-            cl[c].sample.n = 1;
-            cl[c].sample.qw[0] = (int)((cl[c].max_q + 7) >> 3), cl[c].sample.tw[0] = (int)((cl[c].max_t + 7) >> 3);
+        if (cl[c].ns == 0) {
+            cl[c].ns = 1;
+            cl[c].qw[0] = (int)((cl[c].max_q + 7) >> 3), cl[c].tw[0] = (int)((cl[c].max_t + 7) >> 3);
         }
-        const int start = cfg.algo == GLOBAL_ && cfg.start == WITH_START_ ? WITHOUT_START_ : cfg.start;
-        const int forced = st.wc_group >= 64 ? 32 : st.wc_group;
-        p.pk_class[c].max_q = cl[c].max_q;
-        p.pk_class[c].fast = pk_plan(cfg.algo, start, true, cl[c].n, cl[c].max_q, cl[c].sample, sms, forced);
-        p.pk_class[c].cmp = pk_plan(cfg.algo, start, false, std::min(cl[c].n, 32 * sms), cl[c].max_q, cl[c].sample, sms, 0);
-        if (p.pk_class[c].fast.group == 0 || p.pk_class[c].cmp.group == 0) return GB_OK;
     }
+    const int start = cfg.algo == GLOBAL_ && cfg.start == WITH_START_ ? WITHOUT_START_ : cfg.start;
+    const int forced = st.wc_group;
+    if (!pk_plan(cfg.algo, start, cl, sms, forced, p.pkp)) return GB_OK;
     if (grow((void **)&ws.pk_defer, &ws.pk_defer_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
     if (!ws.pk_q && dev_malloc((void **)&ws.pk_q, PK_QUEUE_WORDS * 4) != cudaSuccess) {
         cudaGetLastError();
         return GB_ERR_ALLOC;
     }
     p.pkc = pk_const(cfg.algo, cfg.sc);
-    p.pk_fill = 16 * sms;
     p.order_on = order;
     p.pk = true;
     return GB_OK;
@@ -328,7 +320,7 @@ static void count_pk_classes(const Plan &p, const DevBatch &b, int p0, int p1, i
         n[0] = p1 - p0;
         return;
     }
-    for (int i = p0; i < p1; i++) n[pk_class_of(b.h_q_len[i])]++;
+    for (int i = p0; i < p1; i++) n[pk_class_of(b.h_q_len[i], b.h_t_len[i])]++;
 }
 
 static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p,
@@ -509,7 +501,7 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
             a.scratch_cols = (uint32_t)cols;
         }
     }
-    if ((p.use_wc || p.pk) && !ws.aux) {
+    if (p.use_wc && !ws.aux) {
         /* the warp-cooperative kernels run on the auxiliary stream: with the
          * launch stream's priority, so a caller's prioritised batch keeps it */
         int prio = 0;
@@ -712,70 +704,32 @@ static int launch_dp_split(int algo, int start, bool second, const Plan &p, DpAr
     return launch_one_thread(algo, start, second, p, a, ws, s);
 }
 
-/* DP over pairs [0, a.n) on the packed kernels, class by class (contiguous
- * ranges of `order`; without one, every pair is class 0's).  With warps enough
- * to fill the GPU the first class with pairs -- the longest queries, with the
- * longest sweeps -- runs on the auxiliary stream beside the others (200k mixed
- * LOCAL pairs: 30.6 against 34 ms one after another).  A smaller batch runs on
- * one stream, classes of the same shape in one launch: its one-warp blocks
- * from two streams at once landed on few SMs (1,000 pairs of 250-2,000 bp:
- * 6.0 against 3.2 ms). */
+/* DP over pairs [0, a.n) on the packed kernels, the classes as contiguous
+ * ranges of `order` (without one, every pair is class 0's); classes 0 and 1
+ * beyond their range warp-cooperative on the auxiliary stream beside them. */
 static int launch_pk(const RunCfg &cfg, const Plan &p, DpArgs a, const uint32_t *order, const int *pk_n, Workspace &ws,
                      cudaStream_t s)
 {
     GB_CUDA(cudaMemsetAsync(ws.pk_q, 0, PK_QUEUE_WORDS * 4, s));
     a.tb_kind = ws.tb_kind;
     if (p.tb && p.pk_wc) GB_CUDA(cudaMemsetAsync(ws.tb_kind, 0, (size_t)a.n, s));
-    int used = 0;
-    long warps = 0;
-    for (int c = 0; c < PK_CLASSES; c++) {
-        if (pk_n[c] == 0) continue;
-        used++;
-        warps += (c == 0 && p.pk_wc) ? p.pk_fill : (long)p.pk_class[c].fast.blocks * p.pk_class[c].fast.warps;
-    }
-    const bool full = warps >= p.pk_fill;
-    const bool fork = used > 1 && full;
-    if (fork) {
+    int n[PK_CLASSES], wc = 0;
+    for (int c = 0; c < PK_CLASSES; c++) n[c] = pk_n[c];
+    if (p.pk_wc) wc = n[0] + n[1], n[0] = n[1] = 0;
+    if (wc > 0) {
         GB_CUDA(cudaEventRecord(ws.fork, s));
         GB_CUDA(cudaStreamWaitEvent(ws.aux, ws.fork, 0));
+        timing_mark(K_DP, true, ws.aux);
+        GB_CUDA(launch_dp_wc(cfg.algo, p.start, p.second, a, order, wc, p.mq8_big, p.mt8_big, p.wc_big, ws.wc_rows,
+                             ws.wc_defer, ws.queue + 12, ws.queue + 16, ws.aux));
+        timing_mark(K_DP, false, ws.aux);
+        GB_CUDA(cudaEventRecord(ws.join, ws.aux));
     }
     const int start = cfg.algo == GLOBAL_ && p.start == WITH_START_ ? WITHOUT_START_ : p.start;
-    bool first = true;
-    for (int c = 0, at = 0; c < PK_CLASSES;) {
-        if (pk_n[c] == 0) {
-            c++;
-            continue;
-        }
-        cudaStream_t on = first && fork ? ws.aux : s;
-        first = false;
-        int n = pk_n[c];
-        timing_mark(K_DP, true, on);
-        if (c == 0 && p.pk_wc) {
-            GB_CUDA(launch_dp_wc(cfg.algo, p.start, p.second, a, order, n, p.mq8_big, p.mt8_big, p.wc_big, ws.wc_rows,
-                                 ws.wc_defer, ws.queue + 12, ws.queue + 16, on));
-            c++;
-        } else {
-            const auto &k = p.pk_class[c];
-            WcLaunch fast = k.fast, cmp = k.cmp;
-            int next = c + 1;
-            for (; !full && next < PK_CLASSES; next++) {
-                const WcLaunch &f = p.pk_class[next].fast;
-                if (pk_n[next] == 0) continue;
-                if (f.group != fast.group || f.warps != fast.warps) break;
-                n += pk_n[next];
-                fast.blocks += f.blocks, cmp.blocks += p.pk_class[next].cmp.blocks;
-            }
-            GB_CUDA(launch_dp_pk(cfg.algo, start, a, p.pkc, order ? order + at : nullptr, n, k.max_q, fast, cmp,
-                                 ws.pk_defer + at, ws.pk_q + 4 * c, on));
-            c = next;
-        }
-        timing_mark(K_DP, false, on);
-        at += n;
-    }
-    if (fork) {
-        GB_CUDA(cudaEventRecord(ws.join, ws.aux));
-        GB_CUDA(cudaStreamWaitEvent(s, ws.join, 0));
-    }
+    timing_mark(K_DP, true, s);
+    GB_CUDA(launch_dp_pk(cfg.algo, start, a, p.pkc, p.pkp, order ? order + wc : nullptr, n, ws.pk_defer, ws.pk_q, s));
+    timing_mark(K_DP, false, s);
+    if (wc > 0) GB_CUDA(cudaStreamWaitEvent(s, ws.join, 0));
     return GB_OK;
 }
 

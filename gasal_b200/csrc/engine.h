@@ -101,12 +101,13 @@ void mix_release_all();
 /* the band entry points' per-stream workspaces (band_api.cu) */
 void band_release_all();
 
-/* The packed kernels run one pair of launches per class of query lengths, a
- * contiguous range of the length order; class c takes queries of at least
- * PK_CLASS_WORDS[c] words (and fewer than class c-1's). */
-constexpr int PK_CLASSES = 5;
-constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {ORDER_CAP_WORDS, 64, 32, 16, 0};
-constexpr int PK_QUEUE_WORDS = 4 * PK_CLASSES;
+/* The packed kernels' classes are contiguous ranges of the length order: class
+ * 0 the pairs of at least ORDER_CAP_WORDS query words and PK_LONG_UNITS units
+ * of DP size (2,560 x 2,560 bases), whose sweeps would outlast the rest of a
+ * launch; class c > 0 the other queries of at least PK_CLASS_WORDS[c] words
+ * (and fewer than class c-1's). */
+constexpr uint32_t PK_LONG_UNITS = 25;
+constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {0, ORDER_CAP_WORDS, 64, 32, 16, 0};
 
 /* The decisions and allocations for one batch (plan_batch), so that
  * enqueue_batch issues stream operations only -- capturable into a graph. */
@@ -131,13 +132,9 @@ struct Plan {
     int fb_blocks = 0;      /* grid of the one-thread ksw launch for handed-back pairs (scratch rows) */
     DpArgs a{};
     bool pk = false;        /* the packed kernels (dp_pk.cuh) run every class but pk_wc's */
-    bool pk_wc = false;     /* ... class 0's values leave their range: it runs warp-cooperative (wc_big) */
+    bool pk_wc = false;     /* ... values of classes 0 and 1 leave their range: those run warp-cooperative (wc_big) */
     PkConst pkc{};
-    struct {
-        uint32_t max_q = 0;
-        WcLaunch fast, cmp;
-    } pk_class[PK_CLASSES];
-    long pk_fill = 0;       /* warps that fill the GPU */
+    PkPlan pkp;
     std::vector<int> pk_n;  /* per range, per class: its pairs */
     std::vector<int> cut;   /* pair ranges [cut[c], cut[c+1]) run one after another */
     std::vector<int> nlong; /* per range: pairs on the warp-cooperative kernel */

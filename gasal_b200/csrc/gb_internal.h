@@ -57,6 +57,7 @@ struct DpArgs {
                                            one slot of scratch_cols words per lane group of the grid */
     int32_t *max_off;                   /* unbanded ksw: largest |column - row| of the cells where the
                                            running maximum rose (ksw_extend2's max_off), or null */
+    uint32_t *stuck;                    /* set when a bounded wait of a kernel ran out */
     uint8_t *tb_kind;                   /* per pair: 1 when its traceback storage holds boundary
                                            checkpoints (dp_pk.cuh) instead of direction tiles */
     uint32_t *defer, *ndefer;           /* warp-cooperative table-scoring launch: pairs it leaves to the
@@ -116,6 +117,13 @@ cudaError_t launch_cigar_text(const uint8_t *cigar, const uint32_t *q_off, const
 /* the length order's classes stop at this many query (and target) words:
  * pairs of at least ORDER_CAP_WORDS query words form the order's prefix */
 constexpr uint32_t ORDER_CAP_WORDS = 127;
+/* ... and are sorted by the DP size in units of 4096 word pairs, up to
+ * ORDER_CAP_WORDS units, largest first */
+__host__ __device__ inline uint32_t order_prefix_units(uint32_t qwords, uint32_t twords)
+{
+    const uint64_t u = ((uint64_t)qwords * twords) >> 12;
+    return u < ORDER_CAP_WORDS ? (uint32_t)u : ORDER_CAP_WORDS;
+}
 
 /* length-binned visiting order (sched.cu): bins = order_bins() words of
  * scratch, order = n words */

@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t work_bin(uint32_t qlen, uint32_t tlen)
      * the DP size qw * tw in classes of 4096 words^2, largest first, so the
      * launches that pull them from a work counter start the longest ones
      * first */
-    if (qw >= cap) return cap - min((uint32_t)(((uint64_t)qw * tw) >> 12), cap);
+    if (qw >= cap) return cap - order_prefix_units(qw, tw);
     const uint32_t tr = min(tw, cap);
     /* descending work -> ascending bin */
     return (uint32_t)(ORDER_BINS - 1) - ((qw << ORDER_BITS) | tr);

@@ -65,7 +65,7 @@ def _check(p, b):
 
 
 @pytest.mark.parametrize("p", MODES, ids=lambda p: p.key())
-@pytest.mark.parametrize("group", [0, 8, 16, 32])
+@pytest.mark.parametrize("group", [0, 8, 16, 32, 64])
 def test_edges_of_words_bands_and_rounds(p, group):
     """Query words and target bands one below, at and one above the virtual
     lanes of every group, and single bases."""
@@ -123,3 +123,17 @@ def test_scores_beyond_the_packed_range(p):
     b = _batch(rng, sizes)
     for match in (7, 10):
         _check(replace(p, match=match, mismatch=8, gap_open=12, gap_extend=2), b)
+
+
+@pytest.mark.parametrize("p", MODES, ids=lambda p: p.key())
+@pytest.mark.parametrize("n", [1, 9, 40])
+def test_few_long_pairs(p, n):
+    """Too few pairs to fill the GPU: several warps share a pair, one round
+    and more, among them queries narrower than the handover between warps
+    and targets that end in each of the group's warps."""
+    rng = np.random.default_rng(n + 10 * p.algo)
+    tl = [9000, 530, 1030, 2100, 4200, 600, 3000, 8200, 70]
+    sizes = [(int(rng.integers(1, 2500)) if k % 4 else 100 + k, tl[k % len(tl)] - int(rng.integers(0, 8)))
+             for k in range(n)]
+    sizes[0] = (2300, 9000)
+    _check(p, _batch(rng, sizes))
