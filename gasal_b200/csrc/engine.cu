@@ -444,8 +444,8 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
         p.ksw_short = st.ksw_groups ? ksw_grp_short(b.h_q_len, b.n) : 0;
         if (grow((void **)&ws.fb, &ws.fb_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
         p.band = cfg.band_w != nullptr || cfg.band_model != nullptr;
+        if (grow((void **)&ws.retry, &ws.retry_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
         if (p.band) {
-            if (grow((void **)&ws.retry, &ws.retry_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
             if (cfg.band_model) {
                 if (grow((void **)&ws.feat, &ws.feat_cap, (size_t)b.n * BAND_FEATS_PAD, 4) != GB_OK)
                     return GB_ERR_ALLOC;
@@ -740,11 +740,12 @@ static int launch_pk(const RunCfg &cfg, const Plan &p, DpArgs a, const uint32_t 
  * counters, [2] handed-back count, [3] refused count, [4..5] computed cells
  * (u64), [6..7] warp work counters of the two length classes, [8..9] the
  * same for the recomputation pass, [10] and [11] the lane-group launches'
- * counters of the two passes. */
+ * counters of the two passes, [20..22] the packed launches' counters and the
+ * count of pairs they leave. */
 static int launch_ksw_split(const RunCfg &cfg, const DevBatch &b, const Plan &p, const uint32_t *order, int n,
                             Workspace &ws, cudaStream_t s)
 {
-    GB_CUDA(cudaMemsetAsync(ws.queue, 0, 64, s));
+    GB_CUDA(cudaMemsetAsync(ws.queue, 0, 128, s));
     unsigned long long *cells = reinterpret_cast<unsigned long long *>(ws.queue + 4);
     timing_mark(K_DP, true, s);
     if (p.band) {
@@ -766,7 +767,7 @@ static int launch_ksw_split(const RunCfg &cfg, const DevBatch &b, const Plan &p,
         /* a length order lists the short pairs last */
         const int split = p.ksw_short <= 0 ? -2 : (order ? n - p.ksw_short : -1);
         GB_CUDA(launch_ksw_wc(p.a, order, n, p.ksw_slots, ws.fb, ws.queue + 2, ws.queue + 6, cells, s, split,
-                              ws.queue + 10));
+                              ws.queue + 10, ws.retry, ws.queue + 20));
     }
     timing_mark(K_DP, false, s);
     DpArgs fa = p.a;

@@ -177,10 +177,18 @@ void ksw_wc_classes(const uint32_t *h_q_len, int n, int slots[2]);
  * for queries of at most 248 bases (31 words), the class launches skipping
  * them; >= 0 the list is length-ordered and its short pairs are exactly
  * list[split, nlist): lane groups take those, the class launches the prefix.
- * gq: the lane-group launch's zeroed work counter. */
+ * gq: the lane-group launch's zeroed work counter.  rest (nlist words) and pq3
+ * (three zeroed words): the packed row kernel runs first, and what it leaves
+ * in rest is what the class launches take. */
 cudaError_t launch_ksw_wc(const DpArgs &a, const uint32_t *list, int nlist, const int slots[2], uint32_t *fb,
                           uint32_t *fbn, uint32_t *wq, unsigned long long *cells, cudaStream_t s, int split = -2,
-                          uint32_t *gq = nullptr);
+                          uint32_t *gq = nullptr, uint32_t *rest = nullptr, uint32_t *pq3 = nullptr);
+/* the packed row kernel (ksw_pk.cu) over one length class: pairs it cannot
+ * take (other codes, values beyond 15 bits; with handback also longer
+ * queries) go to rest, counted in *nrest */
+bool ksw_pk_scores_ok(const Scores &sc);
+cudaError_t launch_ksw_pk(const DpArgs &a, const uint32_t *list, int nlist, int slots, int q_lo, bool handback,
+                          uint32_t *rest, uint32_t *nrest, uint32_t *wq, unsigned long long *cells, cudaStream_t s);
 /* pairs with at most 31 query words (the lane-group launch's) */
 int ksw_grp_short(const uint32_t *h_q_len, int n);
 /* The same with a band: pair p is computed within half-width band_w[p]

@@ -899,16 +899,26 @@ static cudaError_t launch_classes(const DpArgs &a, const uint32_t *list, int nli
 
 cudaError_t launch_ksw_wc(const DpArgs &a, const uint32_t *list, int nlist, const int slots[2], uint32_t *fb,
                           uint32_t *fbn, uint32_t *wq, unsigned long long *cells, cudaStream_t s, int split,
-                          uint32_t *gq)
+                          uint32_t *gq, uint32_t *rest, uint32_t *pq3)
 {
     BandArgs ba{nullptr, nullptr, nullptr, cells, 0, 1};
-    if (split < -1) return launch_classes(a, list, nlist, slots, fb, fbn, wq, ba, false, s);
-    /* short queries on lane groups: the order's suffix [split, nlist), or
-     * every pair of an unordered list skipping the longer ones */
-    const cudaError_t e = launch_grp(a, list, nlist, split, fb, fbn, gq, cells, s);
+    int nlong = nlist, q_lo = 0;
+    if (split >= -1) {
+        /* short queries on lane groups: the order's suffix [split, nlist), or
+         * every pair of an unordered list skipping the longer ones */
+        const cudaError_t e = launch_grp(a, list, nlist, split, fb, fbn, gq, cells, s);
+        if (e != cudaSuccess) return e;
+        if (split >= 0) nlong = split;
+        else q_lo = GRP_QMAX + 1;
+    }
+    if (!rest || !ksw_pk_scores_ok(a.sc)) return launch_classes(a, list, nlong, slots, fb, fbn, wq, ba, false, s, q_lo);
+    cudaError_t e = launch_ksw_pk(a, list, nlong, slots[0], q_lo, slots[1] == 0, rest, pq3 + 2, pq3, cells, s);
+    if (e == cudaSuccess && slots[1] > 0)
+        e = launch_ksw_pk(a, list, nlong, slots[1], slots[0] - 1, true, rest, pq3 + 2, pq3 + 1, cells, s);
     if (e != cudaSuccess) return e;
-    if (split >= 0) return launch_classes(a, list, split, slots, fb, fbn, wq, ba, false, s);
-    return launch_classes(a, list, nlist, slots, fb, fbn, wq, ba, false, s, GRP_QMAX + 1);
+    DpArgs r = a;
+    r.n_dev = pq3 + 2;
+    return launch_classes(r, rest, nlong, slots, fb, fbn, wq, ba, false, s, q_lo);
 }
 
 int ksw_grp_short(const uint32_t *h_q_len, int n)
