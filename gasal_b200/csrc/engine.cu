@@ -240,9 +240,7 @@ static int pk_class_of(uint32_t qlen, uint32_t tlen)
 {
     const uint32_t words = (qlen + 7) >> 3;
     if (words >= ORDER_CAP_WORDS) return order_prefix_units(words, (tlen + 7) >> 3) >= PK_LONG_UNITS ? 0 : 1;
-    int c = 2;
-    while (words < PK_CLASS_WORDS[c]) c++;
-    return c;
+    return 2 + (words < PK_CLASS_WORDS[2]) + (words < PK_CLASS_WORDS[3]) + (words < PK_CLASS_WORDS[4]);
 }
 
 /* Whether the packed kernels take this batch, and with what shapes.  They run
@@ -273,6 +271,7 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
             c.qw[c.ns] = (int)((ql + 7) >> 3), c.tw[c.ns] = (int)((tl + 7) >> 3), c.ns++;
         }
     }
+    for (int c = 0; c < PK_CLASSES; c++) p.pk_all[c] = cl[c].n;
     /* an unordered batch is one class: equal lengths, or too few pairs for the order to matter */
     const bool order = b.n >= st.min_order_pairs || (b.n > 64 && st.min_order_pairs <= (1 << 29) && max_q > min_q + min_q / 2);
     if (!order) {
@@ -318,6 +317,10 @@ static void count_pk_classes(const Plan &p, const DevBatch &b, int p0, int p1, i
 {
     if (!p.order_on) {
         n[0] = p1 - p0;
+        return;
+    }
+    if (p1 - p0 == b.n) { /* counted already */
+        std::copy(p.pk_all, p.pk_all + PK_CLASSES, n);
         return;
     }
     for (int i = p0; i < p1; i++) n[pk_class_of(b.h_q_len[i], b.h_t_len[i])]++;
@@ -867,7 +870,11 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
             t.kind = ws.tb_kind, t.order = ord;
             t.pq = b.pq, t.pt = b.pt, t.t_off = ca.t_off;
             t.c0 = p.pkc.c0, t.pa = p.pkc.a, t.pb = p.pkc.b;
-            GB_CUDA(launch_traceback_points(t, s));
+            /* 8 lanes to the pairs whose walks would outlast the rest: queries of 127+ words,
+             * and the longest of any batch while its threads leave the GPU idle */
+            const int *pn = p.pk_n.data() + PK_CLASSES * c;
+            const int longest = p.order_on ? pn[0] + pn[1] : 0;
+            GB_CUDA(launch_traceback_points(t, std::max(longest, TB_COOP_PAIRS), s));
         }
         if (!p.pk || p.pk_wc) GB_CUDA(launch_traceback(t, s));
         timing_mark(K_TB, false, s);

@@ -106,6 +106,7 @@ void band_release_all();
  * of DP size (2,560 x 2,560 bases), whose sweeps would outlast the rest of a
  * launch; class c > 0 the other queries of at least PK_CLASS_WORDS[c] words
  * (and fewer than class c-1's). */
+constexpr int TB_COOP_PAIRS = 8192;
 constexpr uint32_t PK_LONG_UNITS = 25;
 constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {0, ORDER_CAP_WORDS, 64, 32, 16, 0};
 
@@ -135,6 +136,7 @@ struct Plan {
     bool pk_wc = false;     /* ... values of classes 0 and 1 leave their range: those run warp-cooperative (wc_big) */
     PkConst pkc{};
     PkPlan pkp;
+    int pk_all[PK_CLASSES] = {}; /* the batch's pairs per class */
     std::vector<int> pk_n;  /* per range, per class: its pairs */
     std::vector<int> cut;   /* pair ranges [cut[c], cut[c+1]) run one after another */
     std::vector<int> nlong; /* per range: pairs on the warp-cooperative kernel */

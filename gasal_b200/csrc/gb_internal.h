@@ -98,8 +98,9 @@ cudaError_t launch_revcomp(uint32_t *pq, uint32_t *pt, const uint32_t *q_off, co
 cudaError_t launch_dp(int algo, int start, bool second, const DpArgs &a, int block, int max_q8,
                       cudaStream_t s);
 cudaError_t launch_traceback(const TbArgs &a, cudaStream_t s);
-/* the pairs whose kind is 1 (LOCAL, GLOBAL): walks over recomputed blocks */
-cudaError_t launch_traceback_points(const TbArgs &a, cudaStream_t s);
+/* the pairs whose kind is 1 (LOCAL, GLOBAL): walks over recomputed blocks, the
+ * first `coop` of a.order on 8 lanes each */
+cudaError_t launch_traceback_points(const TbArgs &a, int coop, cudaStream_t s);
 
 /* Lets a kernel use the most dynamic shared memory the device gives a block
  * (set once per kernel and device).  Kernels launched with different sizes
