@@ -567,8 +567,9 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
     /* tile budget: the setting, but at most half of the device memory that is
      * free or already held as this stream's tiles (fewer, longer chunks on a
      * large device; room left for other streams) */
-    uint64_t budget_bytes = st.tb_budget_bytes;
-    {
+    uint64_t budget_bytes = st.tb_budget_bytes, all = 0;
+    for (int i = 0; i < b.n; i++) all += tb_tiles(b.h_q_len[i], b.h_t_len[i]);
+    if (all > ws.tb_cap) { /* a batch that fits what is held needs no look at the device's memory */
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
             const uint64_t avail = ((uint64_t)free_b + (uint64_t)ws.tb_cap * 16) / 2;
@@ -802,10 +803,7 @@ int enqueue_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspa
     /* pack and reverse/complement */
     if (!cfg.is_packed) {
         timing_mark(K_PACK, true, s);
-        GB_CUDA(launch_pack(b.q, b.q_bytes, b.pq, s));
-        timing_mark(K_PACK, false, s);
-        timing_mark(K_PACK, true, s);
-        GB_CUDA(launch_pack(b.t, b.t_bytes, b.pt, s));
+        GB_CUDA(launch_pack2(b.q, b.q_bytes, b.pq, b.t, b.t_bytes, b.pt, s));
         timing_mark(K_PACK, false, s);
     }
     if (cfg.reverse_complement) {
@@ -837,6 +835,7 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
                                ws, s);
     }
     GB_CUDA(cudaMemcpyAsync(ws.d_tb_off, ws.h_tb_off, (size_t)b.n * 8, cudaMemcpyHostToDevice, s));
+    if (p.mark_tb_off) GB_CUDA(cudaEventRecord(ws.tb_off_free, s)); /* the pinned offsets may be written again */
     for (size_t c = 0; c + 1 < p.cut.size(); c++) {
         const int p0 = p.cut[c], p1 = p.cut[c + 1];
         DpArgs ca = p.a;
@@ -887,8 +886,8 @@ int run_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &
     Plan p;
     int rc = plan_batch(cfg, b, o, ws, p, s);
     if (rc != GB_OK) return rc;
+    p.mark_tb_off = true;
     rc = enqueue_batch(cfg, b, o, ws, p, s);
-    if (rc == GB_OK && p.tb) GB_CUDA(cudaEventRecord(ws.tb_off_free, s));
     return rc;
 }
 

@@ -114,6 +114,7 @@ constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {0, ORDER_CAP_WORDS, 64, 32, 16,
  * enqueue_batch issues stream operations only -- capturable into a graph. */
 struct Plan {
     bool tb = false, second = false, use_wc = false, order_on = false;
+    bool mark_tb_off = false;    /* enqueue_batch records tb_off_free itself (not under capture) */
     int start = 0, block = 64, mq8 = 0, mt8 = 0;
     uint32_t wc_min_q = 0;
     WcLaunch wc;                 /* shape of the warp-cooperative launch */

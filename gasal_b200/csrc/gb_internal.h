@@ -92,6 +92,9 @@ struct TbArgs {
 
 /* ---- launchers (stream-ordered, no allocation) ---- */
 cudaError_t launch_pack(const uint8_t *ascii, uint32_t nbytes, uint32_t *words, cudaStream_t s);
+/* both sides of a batch in one launch */
+cudaError_t launch_pack2(const uint8_t *q, uint32_t q_bytes, uint32_t *pq, const uint8_t *t, uint32_t t_bytes,
+                         uint32_t *pt, cudaStream_t s);
 cudaError_t launch_revcomp(uint32_t *pq, uint32_t *pt, const uint32_t *q_off, const uint32_t *t_off,
                            const uint32_t *q_len, const uint32_t *t_len, const uint8_t *q_op,
                            const uint8_t *t_op, int32_t n, int ref_reverse, cudaStream_t s);

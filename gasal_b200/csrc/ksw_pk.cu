@@ -26,6 +26,10 @@
  *   row is only cut where its entries are 0), so a row's last tile stores 0
  *   there instead of leaving them.
  *
+ * Measured on a B200 against ksw_wc.cu's kernel: 50k pairs of 250-2,000 bp 44.2
+ * to 30.8 ms, 200k of 50-5,000 bp 57.7 to 40.9 ms (lane groups for the short
+ * ones in both); about 400 instructions per row, the integer pipe at 70%.
+ *
  * Takes pairs of plain codes whose largest value times match + 1 fits 15 bits;
  * the others go to a list for ksw_wc.cu's kernels.
  */

@@ -30,14 +30,27 @@ __device__ __forceinline__ uint32_t pack8(uint32_t lo, uint32_t hi)
     return ((ev << 4) & 0xF0F0F0F0u) | (od & 0x0F0F0F0Fu);
 }
 
-__global__ void __launch_bounds__(256) pack_kernel(const uint8_t *__restrict__ ascii, uint32_t nbytes,
-                                                   uint32_t *__restrict__ words)
+/* One side's range, by the blocks [first, first + nblocks) of the launch: a
+ * batch's queries and targets are packed by one launch (a second one was 3 of
+ * the 120 us of a 64-pair call). */
+struct PackSide {
+    const uint8_t *ascii;
+    uint32_t *words;
+    uint32_t nbytes;
+};
+
+__global__ void __launch_bounds__(256) pack_kernel(PackSide q, PackSide t, uint32_t q_blocks)
 {
+    const bool second = blockIdx.x >= q_blocks;
+    const uint8_t *__restrict__ ascii = second ? t.ascii : q.ascii;
+    uint32_t *__restrict__ words = second ? t.words : q.words;
+    const uint32_t nbytes = second ? t.nbytes : q.nbytes;
+    const uint32_t block = second ? blockIdx.x - q_blocks : blockIdx.x;
     const uint32_t n32 = nbytes >> 5; /* 32-byte chunks */
-    const uint32_t stride = gridDim.x * blockDim.x;
+    const uint32_t stride = (second ? gridDim.x - q_blocks : q_blocks) * blockDim.x;
     const uint4 *in = reinterpret_cast<const uint4 *>(ascii);
     uint4 *out = reinterpret_cast<uint4 *>(words);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n32; i += stride) {
+    for (uint32_t i = block * blockDim.x + threadIdx.x; i < n32; i += stride) {
         const uint4 a = __ldcs(in + 2 * i);
         const uint4 b = __ldcs(in + 2 * i + 1);
         uint4 w;
@@ -49,25 +62,32 @@ __global__ void __launch_bounds__(256) pack_kernel(const uint8_t *__restrict__ a
     }
     /* tail: up to three 8-byte groups */
     const uint32_t done = n32 << 2, total = nbytes >> 3;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < total - done) {
-        const uint2 v = reinterpret_cast<const uint2 *>(ascii)[done + t];
-        words[done + t] = pack8(v.x, v.y);
+    const uint32_t x = block * blockDim.x + threadIdx.x;
+    if (x < total - done) {
+        const uint2 v = reinterpret_cast<const uint2 *>(ascii)[done + x];
+        words[done + x] = pack8(v.x, v.y);
     }
+}
+
+cudaError_t launch_pack2(const uint8_t *q, uint32_t q_bytes, uint32_t *pq, const uint8_t *t, uint32_t t_bytes,
+                         uint32_t *pt, cudaStream_t s)
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto blocks_of = [&](uint32_t nbytes) {
+        const uint32_t blocks = ((nbytes >> 5) + 1 + 255) / 256, cap = (uint32_t)sms * 8;
+        return nbytes == 0 ? 0u : blocks < cap ? blocks : cap;
+    };
+    const uint32_t bq = blocks_of(q_bytes), bt = blocks_of(t_bytes);
+    if (bq + bt == 0) return cudaSuccess;
+    pack_kernel<<<bq + bt, 256, 0, s>>>(PackSide{q, pq, q_bytes}, PackSide{t, pt, t_bytes}, bq);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_pack(const uint8_t *ascii, uint32_t nbytes, uint32_t *words, cudaStream_t s)
 {
-    if (nbytes == 0) return cudaSuccess;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t chunks = (nbytes >> 5) + 1;
-    uint32_t blocks = (chunks + 255) / 256;
-    const uint32_t cap = (uint32_t)sms * 8;
-    if (blocks > cap) blocks = cap;
-    pack_kernel<<<blocks, 256, 0, s>>>(ascii, nbytes, words);
-    return cudaGetLastError();
+    return launch_pack2(ascii, nbytes, words, nullptr, 0, nullptr, s);
 }
 
 __device__ __forceinline__ uint32_t nib_reverse(uint32_t x)
