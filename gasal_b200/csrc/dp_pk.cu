@@ -202,9 +202,11 @@ bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPl
         }
     }
     if (p.warps == 0) return false;
-    p.cmp_cols = ring_words(8, max_q);
-    const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1, (size_t)p.cmp_cols * 16);
-    p.cmp_blocks = std::min((n + 3) / 4, std::max(sms * res, sms));
+    p.cmp_cols[0] = max_q >= (uint32_t)PK_CMP_LONG ? ring_words(32, max_q) : 0;
+    p.cmp_cols[1] = ring_words(4, std::min(max_q, (uint32_t)PK_CMP_LONG - 1));
+    const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1,
+                                   (size_t)std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]) * 4);
+    p.cmp_blocks = std::min(p.cmp_cols[0] ? n : (n + 7) / 8, std::max(sms * res, sms));
     return res > 0;
 }
 
@@ -232,16 +234,17 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     /* the table-scoring launch, then the compare-scoring one over the pairs it
      * left (a target with another code than A, C, G, T, N) */
     DpArgs f = a;
-    f.queue = wq, f.defer = defer, f.ndefer = wq + PK_CLASSES + 1, f.n_dev = nullptr, f.stuck = wq + PK_CLASSES + 2;
+    f.queue = wq, f.defer = defer, f.ndefer = wq + PK_CLASSES + 2, f.n_dev = nullptr, f.stuck = wq + PK_CLASSES + 4;
     cudaError_t e = launch(p.warps == 4 ? PK_W4 : p.warps == 2 ? PK_W2 : PK_W1, f, cl, list,
                            (int)std::min<long>((warps + p.warps - 1) / p.warps, p.blocks), p.warps);
     if (e != cudaSuccess) return e;
     DpArgs c = f;
     c.queue = wq + PK_CLASSES, c.defer = nullptr, c.ndefer = nullptr, c.n_dev = f.ndefer;
-    PkClasses one;
-    one.n = 1, one.warp_words = 4 * p.cmp_cols;
-    one.k[0] = {8, 0, total, p.cmp_cols};
-    return launch(PK_CMP, c, one, defer, std::min((total + 3) / 4, p.cmp_blocks), 1);
+    PkClasses left;
+    left.warp_words = std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]);
+    if (p.cmp_cols[0]) left.k[left.n++] = {32, 0, total, p.cmp_cols[0]};
+    left.k[left.n++] = {4, 0, total, p.cmp_cols[1]};
+    return launch(PK_CMP, c, left, defer, std::min(total, p.cmp_blocks), 1);
 }
 
 } // namespace gb

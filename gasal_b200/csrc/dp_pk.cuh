@@ -40,6 +40,15 @@
  * the group virtual lanes, and the ring holds a whole one, so the last warp
  * never waits for room.
  *
+ * Measured on a B200 (us a batch, before with one pair per thread below 32
+ * query words and one band per lane above, after): 300k SEMI_GLOBAL 150 bp with
+ * starts 6,960 / 4,710; 200k LOCAL of 50-5,000 bp with starts 51,700 / 27,000;
+ * 150k SEMI_GLOBAL of the same lengths 39,400 / 19,000; 100k GLOBAL of
+ * 50-1,000 bp with traceback 19,000 / 6,400; 5k GLOBAL 150 bp 460 / 135; 1k
+ * LOCAL of 250-2,000 bp 750,000 / 2,860.  Rates on equal lengths of 500: GLOBAL
+ * 5.1 T cells/s, SEMI_GLOBAL 4.2, LOCAL 3.6.  A LOCAL step of a warp is about 700 instructions, 500 of
+ * them on that pipe (73% busy at two warps a scheduler).
+ *
  * H and E cross a band boundary as 16-bit values, as in the reference's short2
  * row buffer; the host only sends pairs here whose values cannot leave 15 bits
  * (pk_fits), so the results are the reference's bit for bit.
@@ -105,14 +114,14 @@ __device__ void pk_score_table(uint2 *tab, const Scores &sc, bool n_zero, int ab
     for (int x = threadIdx.x; x < 256; x += blockDim.x) tab[x] = make_uint2(row(x >> 4), row(x & 15));
 }
 
-/* The pairs list[0..nl) on G lanes of W warps each, taken from the zeroed
+/* The pairs list[0], list[dir], .. (nl of them) on G lanes of W warps each, taken from the zeroed
  * counter `queue`.  smem: the warp's rings (W > 1: the block's).
  * FAST: targets of A, C, G, T and N, scores by one prmt per packed cell (its
  * selector's bytes: the row's class, then that byte's sign).  Otherwise
  * compares, any code. */
 template <int G, int W, int ALGO, int START, bool FAST>
 __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, const uint2 *tab, uint32_t *pk_smem,
-                                         const uint32_t *list, int nl, uint32_t *queue, int ring_cols)
+                                         const uint32_t *list, int nl, uint32_t *queue, int ring_cols, int dir = 1)
 {
     constexpr int LANES = G * W;
     constexpr int V = 2 * G;
@@ -151,7 +160,7 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
         if ((int)item0 >= nl) break;
         const int item = (int)item0 + lane / G;
         const bool listed = item < nl;
-        const int i = listed ? (list ? (int)list[item] : item) : 0;
+        const int i = listed ? (list ? (int)list[dir * item] : item) : 0;
         const int qlen0 = listed ? (int)A.q_len[i] : 0, tlen0 = listed ? (int)A.t_len[i] : 0;
         const uint32_t *q = A.pq + (listed ? (A.q_off[i] >> 3) : 0);
         const uint32_t *t = A.pt + (listed ? (A.t_off[i] >> 3) : 0);
@@ -171,7 +180,11 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
                 with_n = W > 1 ? group_any(odd & 6u) : __any_sync(0xFFFFFFFFu, odd & 6u);
             }
             if (group_any(bad)) {
-                if (listed && gl == 0 && wi == 0) A.defer[atomicAdd(A.ndefer, 1u)] = (uint32_t)i;
+                /* left to compare scoring: short pairs from the list's front, long ones from its end */
+                if (listed && gl == 0 && wi == 0) {
+                    if (qlen0 >= PK_CMP_LONG) A.defer[A.n - 1 - (int)atomicAdd(A.ndefer + 1, 1u)] = (uint32_t)i;
+                    else A.defer[atomicAdd(A.ndefer, 1u)] = (uint32_t)i;
+                }
                 has = false;
             }
         }
@@ -703,10 +716,13 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
     for (int c = 0; c < C.n; c++) {
         const PkClass &k = C.k[c];
         const uint32_t *l = list ? list + k.first : nullptr;
-        const int nl = A.n_dev ? min((int)*A.n_dev, k.n) : k.n;
+        [[maybe_unused]] const int nl = k.n;
         uint32_t *qu = A.queue + c;
-        if (!FAST) {
-            pk_pairs<8, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols);
+        if constexpr (!FAST) { /* what the table-scoring launch left: long pairs, then short ones */
+            if (k.group == 32)
+                pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l + (A.n - 1), (int)A.n_dev[1], qu, k.ring_cols, -1);
+            else
+                pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols);
             continue;
         }
         switch (k.group) {

@@ -44,7 +44,10 @@ struct PkClasses {
 };
 
 using PkKernel = void (*)(DpArgs, PkConst, PkClasses, const uint32_t *);
-/* compare scoring (8 lanes to a pair); table scoring in blocks of 1, 2, 4 warps */
+/* compare scoring takes queries of PK_CMP_LONG bases on 32 lanes, shorter ones
+ * on 4 (100k SEMI_GLOBAL 150 bp pairs with such targets: 8 lanes 4.1 ms) */
+constexpr int PK_CMP_LONG = 64 * 8;
+/* compare scoring; table scoring in blocks of 1, 2, 4 warps */
 enum PkVariant { PK_CMP, PK_W1, PK_W2, PK_W4, PK_VARIANTS };
 PkKernel pk_kernel_local(PkVariant v, int start);
 PkKernel pk_kernel_global(PkVariant v, int start);
@@ -63,7 +66,7 @@ struct PkPlan {
     int group[PK_CLASSES] = {};
     int ring_cols[PK_CLASSES] = {};
     int warp_words = 0, warps = 0, blocks = 0;         /* blocks: most that are resident */
-    int cmp_cols = 0, cmp_blocks = 0;
+    int cmp_cols[2] = {}, cmp_blocks = 0;              /* compare scoring: long pairs (32 lanes), short ones (4) */
 };
 
 /* The packed kernels take LOCAL, GLOBAL and target-tail SEMI_GLOBAL without a
@@ -77,7 +80,7 @@ PkConst pk_const(int algo, const Scores &sc);
 bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPlan &p);
 /* n[c]: the pairs of class c, in list order.  wq: PK_QUEUE_WORDS zeroed words;
  * defer: a word per pair */
-constexpr int PK_QUEUE_WORDS = PK_CLASSES + 3;
+constexpr int PK_QUEUE_WORDS = PK_CLASSES + 5;
 cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const PkPlan &p, const uint32_t *list,
                          const int *n, uint32_t *defer, uint32_t *wq, cudaStream_t s);
 

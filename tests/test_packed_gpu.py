@@ -82,8 +82,8 @@ def test_edges_of_words_bands_and_rounds(p, group):
 @pytest.mark.parametrize("odd", [b"N", b"NR", b"Nn", b"RYK"], ids=["N", "N+R", "N+n", "IUPAC"])
 def test_other_codes(p, odd):
     rng = np.random.default_rng(len(odd) + 7 * p.algo)
-    _check(p, _batch(rng, [(int(q), int(q) + int(d)) for q, d in zip(rng.integers(5, 300, 90), rng.integers(-4, 60, 90))],
-                     odd=odd))
+    sizes = [(int(q), int(q) + int(d)) for q, d in zip(rng.integers(5, 300, 90), rng.integers(-4, 60, 90))]
+    _check(p, _batch(rng, sizes + [(511, 530), (512, 520), (1300, 1200), (900, 2100), (2000, 2050)], odd=odd))
 
 
 SCORES = [dict(match=2, mismatch=3, gap_open=5, gap_extend=2), dict(match=1, mismatch=1, gap_open=0, gap_extend=1),
