@@ -152,6 +152,7 @@ void release_workspace(Workspace &w)
     if (w.pk_defer) cudaFree(w.pk_defer);
     if (w.pk_q) cudaFree(w.pk_q);
     if (w.tb_kind) cudaFree(w.tb_kind);
+    if (w.words) cudaFree(w.words);
     if (w.aux) cudaStreamDestroy(w.aux);
     if (w.queue) cudaFree(w.queue);
     if (w.fork) cudaEventDestroy(w.fork);
@@ -324,6 +325,21 @@ static void count_pk_classes(const Plan &p, const DevBatch &b, int p0, int p1, i
         return;
     }
     for (int i = p0; i < p1; i++) n[pk_class_of(b.h_q_len[i], b.h_t_len[i])]++;
+}
+
+/* Words of a packed side to copy before the first walk (0: none).  A caller may
+ * pass a CIGAR buffer that the packed words lie in: a storage with isPacked has
+ * one query buffer for both.  CIGARs land at each pair's byte offset, words at
+ * half of it, so one pair's CIGAR covers other pairs' words -- which the
+ * checkpoint walk reads while it writes, and the sweep of a later chunk after
+ * it.  (Direction tiles of a single chunk need no words: no copy.)
+ * A side packed by the caller fills the buffer it came in. */
+static size_t words_under_cigars(const RunCfg &cfg, const DevOut &o, uint32_t cigar_bytes, const uint8_t *side,
+                                 uint32_t bytes, const uint32_t *words)
+{
+    const size_t n = cfg.is_packed && (const void *)side == (const void *)words ? bytes / 4 : bytes / 8;
+    const uintptr_t c = (uintptr_t)o.cigar, w = (uintptr_t)words;
+    return o.cigar && words && c < w + 4 * n && w < c + cigar_bytes ? n : 0;
 }
 
 static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p,
@@ -611,6 +627,14 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
         }
         max_chunk = std::max(max_chunk, (size_t)(p1 - p0));
     }
+    if (p.pk || p.cut.size() > 2) {
+        p.copy_q = words_under_cigars(cfg, o, b.q_bytes, b.q, b.q_bytes, b.pq);
+        p.copy_t = words_under_cigars(cfg, o, b.q_bytes, b.t, b.t_bytes, b.pt);
+        const size_t words = ((p.copy_q + 31) & ~(size_t)31) + p.copy_t;
+        if (words > 0 && grow((void **)&ws.words, &ws.words_cap, words, 4) != GB_OK) return GB_ERR_ALLOC;
+        if (p.copy_q) a.pq = ws.words;
+        if (p.copy_t) a.pt = ws.words + ((p.copy_q + 31) & ~(size_t)31);
+    }
     if (!p.pk) p.order_on = p.use_wc || b.n >= st.min_order_pairs;
     if (p.pk && grow((void **)&ws.tb_kind, &ws.tb_kind_cap, max_chunk, 1) != GB_OK) return GB_ERR_ALLOC;
     if (p.order_on && ensure_order_buffers(ws, max_chunk) != GB_OK) return GB_ERR_ALLOC;
@@ -835,6 +859,9 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
                                ws, s);
     }
     GB_CUDA(cudaMemcpyAsync(ws.d_tb_off, ws.h_tb_off, (size_t)b.n * 8, cudaMemcpyHostToDevice, s));
+    if (p.copy_q) GB_CUDA(cudaMemcpyAsync(ws.words, b.pq, p.copy_q * 4, cudaMemcpyDeviceToDevice, s));
+    if (p.copy_t)
+        GB_CUDA(cudaMemcpyAsync(const_cast<uint32_t *>(p.a.pt), b.pt, p.copy_t * 4, cudaMemcpyDeviceToDevice, s));
     if (p.mark_tb_off) GB_CUDA(cudaEventRecord(ws.tb_off_free, s)); /* the pinned offsets may be written again */
     for (size_t c = 0; c + 1 < p.cut.size(); c++) {
         const int p0 = p.cut[c], p1 = p.cut[c + 1];
@@ -867,7 +894,7 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
         timing_mark(K_TB, true, s);
         if (p.pk) {
             t.kind = ws.tb_kind, t.order = ord;
-            t.pq = b.pq, t.pt = b.pt, t.t_off = ca.t_off;
+            t.pq = ca.pq, t.pt = ca.pt, t.t_off = ca.t_off;
             t.c0 = p.pkc.c0, t.pa = p.pkc.a, t.pb = p.pkc.b;
             /* 8 lanes to the pairs whose walks would outlast the rest: queries of 127+ words,
              * and the longest of any batch while its threads leave the GPU idle */

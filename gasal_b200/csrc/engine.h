@@ -75,6 +75,8 @@ struct Workspace {
     uint32_t *pk_q = nullptr;    /* PK_QUEUE_WORDS counters of the packed launches */
     uint8_t *tb_kind = nullptr;  /* per pair of a traceback chunk: 1 = boundary checkpoints, 0 = direction tiles */
     size_t tb_kind_cap = 0;
+    uint32_t *words = nullptr;   /* copies of packed words that CIGARs are written over */
+    size_t words_cap = 0;
     uint32_t *order2 = nullptr;  /* visiting order of the separate start passes */
     size_t order2_cap = 0;
     uint32_t *bins = nullptr;    /* order_bins() class counters */
@@ -139,6 +141,9 @@ struct Plan {
     PkPlan pkp;
     int pk_all[PK_CLASSES] = {}; /* the batch's pairs per class */
     std::vector<int> pk_n;  /* per range, per class: its pairs */
+    /* packed words (query, target) that lie where the CIGARs are written and are
+     * still read after the first of them: those batches read a copy */
+    size_t copy_q = 0, copy_t = 0;
     std::vector<int> cut;   /* pair ranges [cut[c], cut[c+1]) run one after another */
     std::vector<int> nlong; /* per range: pairs on the warp-cooperative kernel */
     std::vector<int> nbig;  /* per range: of those, the leading ORDER_CAP_WORDS+ word ones */
