@@ -73,7 +73,8 @@ bool pk_scores_ok(int algo, const Scores &sc)
 }
 
 /* Every value of the sweep must stay within the 15 bits of its half.  LOCAL:
- * the column key 4*H + 4*b*(bc+1) + 3.  GLOBAL / SEMI_GLOBAL: H lies between
+ * the column key 4*H + 4*b*(bc+1) + 3 <= 32767.  max_min counts whole words: a
+ * LOCAL sweep scores what follows a sequence in its last word.  GLOBAL / SEMI_GLOBAL: H lies between
  * the all-gap path, at least -(2o + e*(q+t) + mismatch), and match*min(q, t);
  * a gap opened from a mismatch below the lower end is the lowest value held. */
 bool pk_fits(int algo, const Scores &sc, uint32_t max_q, uint32_t max_t, uint32_t max_min)
@@ -82,7 +83,7 @@ bool pk_fits(int algo, const Scores &sc, uint32_t max_q, uint32_t max_t, uint32_
     if (q8 > 12000 || t8 > 65528) return false;
     const int64_t top = (int64_t)sc.match * max_min;
     const int ab8 = 9 * (sc.e + b_of(algo, sc));
-    if (algo == LOCAL_) return top <= 8100 - 8 * sc.e;
+    if (algo == LOCAL_) return top <= 8191 - 8 * sc.e;
     const int64_t low = 3 * (int64_t)sc.o + 4 * (int64_t)sc.mismatch +
                         (int64_t)sc.e * (std::max<int64_t>(q8, 512) + t8 + 64) + ab8 + 256;
     return low <= C0_SIGNED - 64 && top + ab8 + sc.match + sc.mismatch <= 32767 - C0_SIGNED - 64;

@@ -53,8 +53,8 @@ PkKernel pk_kernel_local(PkVariant v, int start);
 PkKernel pk_kernel_global(PkVariant v, int start);
 PkKernel pk_kernel_semi(PkVariant v, int start);
 
-/* lengths of the pairs of one class: their number, the longest, and (words)
- * up to 128 of them */
+/* lengths of the pairs of one class: their number, the longest query, target
+ * and min(query, target) in whole words (8 bases), and (words) up to 128 of them */
 struct PkLengths {
     int n = 0;
     uint32_t max_q = 0, max_t = 0, max_min = 0;
@@ -72,7 +72,7 @@ struct PkPlan {
 /* The packed kernels take LOCAL, GLOBAL and target-tail SEMI_GLOBAL without a
  * second best (SEMI_GLOBAL: without a traceback): scores of pk_scores_ok, and
  * pairs whose longest query, longest target and longest min(query, target)
- * keep every value within 15 bits (pk_fits). */
+ * (in whole words) keep every value within 15 bits (pk_fits). */
 bool pk_scores_ok(int algo, const Scores &sc);
 bool pk_fits(int algo, const Scores &sc, uint32_t max_q, uint32_t max_t, uint32_t max_min);
 PkConst pk_const(int algo, const Scores &sc);

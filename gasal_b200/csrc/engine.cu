@@ -265,7 +265,8 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
         const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
         PkLengths &c = cl[pk_class_of(ql, tl)];
         c.n++;
-        c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl), c.max_min = std::max(c.max_min, std::min(ql, tl));
+        c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl);
+        c.max_min = std::max(c.max_min, (std::min(ql, tl) + 7) & ~7u); /* bytes after the end may be bases, and score */
         min_q = std::min(min_q, ql), max_q = std::max(max_q, ql);
         if (i >= next && c.ns < 128) {
             next += stride;
