@@ -376,7 +376,10 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
     const uint32_t big_q = ORDER_CAP_WORDS * 8 - 7;
     /* a pair needs at least as many query words as its lane group (the
      * group's ring reader must trail its writer) */
-    const int min_words = std::max(st.wc_min_qregs, st.wc_group > 0 ? st.wc_group : 8);
+    /* pairs of ORDER_CAP_WORDS+ query words lead the length order by DP size, not by
+     * query length: a higher threshold could not tell them apart there */
+    const int min_words =
+        std::min(std::max(st.wc_min_qregs, st.wc_group > 0 ? st.wc_group : 8), (int)ORDER_CAP_WORDS);
     p.wc_min_q = (uint32_t)min_words * 8 - 7;
     for (int i = 0; i < b.n && (!p.pk || p.pk_wc); i++) {
         const uint32_t ql = b.h_q_len[i];

@@ -274,8 +274,9 @@ int gb_graph_stats(int64_t *counts);
 /* Launch tuning (no reference counterpart).  block: threads per block of the
  * one-pair-per-thread DP kernel (32, 64 or 128); wc_min_qregs: pairs
  * whose query has at least this many 8-base words run warp-cooperative
- * (LOCAL/GLOBAL/target-tail SEMI_GLOBAL; at least 8, and never fewer than
- * wc_group, which that kernel needs); min_order_pairs: batches with at least this many pairs are
+ * (LOCAL/GLOBAL/target-tail SEMI_GLOBAL; at least 8, never fewer than
+ * wc_group, which that kernel needs, and more than 127 count as 127);
+ * min_order_pairs: batches with at least this many pairs are
  * visited length-binned.  Results never depend on these. */
 typedef struct {
     int32_t block;
