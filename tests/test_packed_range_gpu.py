@@ -40,13 +40,19 @@ def _equal_pairs(rng, n):
 
 @pytest.mark.parametrize("p", MODES, ids=lambda p: p.key())
 @pytest.mark.parametrize("match,lengths", [(50, range(153, 169)), (16, range(497, 514)), (59, range(265, 283)),
-                                           (13, (617, 624, 625, 632)), (1, (8176, 8177))], ids=lambda v: v if isinstance(v, int) else "")
+                                           (13, (617, 624, 625, 632))], ids=lambda v: v if isinstance(v, int) else "")
 def test_highest_scores(p, match, lengths):
     """match * length crosses 8,183 (LOCAL) or about 16,200 (the others) among
     the lengths, by the bases counted or by those after the end."""
     rng = np.random.default_rng(match)
     for n in lengths:
         _check(replace(p, match=match), _equal_pairs(rng, n), f"{p.key()} match {match} length {n}")
+
+
+@pytest.mark.parametrize("n", [8176, 8177])
+def test_highest_scores_of_long_pairs(n):
+    p = Params(algo=LOCAL)
+    _check(p, _equal_pairs(np.random.default_rng(n), n), f"length {n}")
 
 
 @pytest.mark.parametrize("p", [m for m in MODES if m.algo != LOCAL], ids=lambda p: p.key())
