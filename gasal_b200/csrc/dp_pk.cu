@@ -198,13 +198,15 @@ bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPl
                     if (cl[c].n) {
                         p.group[c] = k[c] == WIDE ? 32 * w : 1 << k[c];
                         p.ring_cols[c] = ring_words(p.group[c], cl[c].max_q);
+                        p.max_q8[c] = (int)((cl[c].max_q + 7) & ~7u);
                     }
             }
         }
     }
     if (p.warps == 0) return false;
-    p.cmp_cols[0] = max_q >= (uint32_t)PK_CMP_LONG ? ring_words(32, max_q) : 0;
-    p.cmp_cols[1] = ring_words(4, std::min(max_q, (uint32_t)PK_CMP_LONG - 1));
+    p.cmp_q8[0] = (int)((max_q + 7) & ~7u), p.cmp_q8[1] = std::min(p.cmp_q8[0], PK_CMP_LONG);
+    p.cmp_cols[0] = p.cmp_q8[0] >= PK_CMP_LONG ? ring_words(32, max_q) : 0;
+    p.cmp_cols[1] = ring_words(4, (uint32_t)p.cmp_q8[1]);
     const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1,
                                    (size_t)std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]) * 4);
     p.cmp_blocks = std::min(p.cmp_cols[0] ? n : (n + 7) / 8, std::max(sms * res, sms));
@@ -220,7 +222,7 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     cl.warp_words = p.warp_words;
     for (int c = 0; c < PK_CLASSES; c++) {
         if (n[c] == 0) continue;
-        cl.k[cl.n++] = {p.group[c], total, n[c], p.ring_cols[c]};
+        cl.k[cl.n++] = {p.group[c], total, n[c], p.ring_cols[c], p.max_q8[c]};
         warps += ((long)n[c] * p.group[c] + 31) / 32;
         total += n[c];
     }
@@ -243,8 +245,8 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     c.queue = wq + PK_CLASSES, c.defer = nullptr, c.ndefer = nullptr, c.n_dev = f.ndefer;
     PkClasses left;
     left.warp_words = std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]);
-    if (p.cmp_cols[0]) left.k[left.n++] = {32, 0, total, p.cmp_cols[0]};
-    left.k[left.n++] = {4, 0, total, p.cmp_cols[1]};
+    if (p.cmp_cols[0]) left.k[left.n++] = {32, 0, total, p.cmp_cols[0], p.cmp_q8[0]};
+    left.k[left.n++] = {4, 0, total, p.cmp_cols[1], p.cmp_q8[1]};
     return launch(PK_CMP, c, left, defer, std::min(total, p.cmp_blocks), 1);
 }
 

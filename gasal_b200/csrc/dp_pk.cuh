@@ -121,7 +121,8 @@ __device__ void pk_score_table(uint2 *tab, const Scores &sc, bool n_zero, int ab
  * compares, any code. */
 template <int G, int W, int ALGO, int START, bool FAST>
 __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, const uint2 *tab, uint32_t *pk_smem,
-                                         const uint32_t *list, int nl, uint32_t *queue, int ring_cols, int dir = 1)
+                                         const uint32_t *list, int nl, uint32_t *queue, int ring_cols, int max_q8,
+                                         int dir = 1)
 {
     constexpr int LANES = G * W;
     constexpr int V = 2 * G;
@@ -162,11 +163,17 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
         const bool listed = item < nl;
         const int i = listed ? (list ? (int)list[dir * item] : item) : 0;
         const int qlen0 = listed ? (int)A.q_len[i] : 0, tlen0 = listed ? (int)A.t_len[i] : 0;
+        /* longer than the host's copy of the lengths said: its ring would not hold it.  Never
+         * written, as in the one-thread kernel (this only guards memory), and not walked */
+        auto too_long = [&]() { return (uint32_t)qlen0 > (uint32_t)max_q8; };
+        auto skip = [&]() {
+            if (TB && gl == 0 && wi == 0) A.tb_kind[i] = 2;
+        };
         const uint32_t *q = A.pq + (listed ? (A.q_off[i] >> 3) : 0);
         const uint32_t *t = A.pt + (listed ? (A.t_off[i] >> 3) : 0);
         bool has = listed, with_n = false;
         if (FAST) {
-            uint32_t odd = 0, odd_q = 0;
+            uint32_t odd = too_long() ? 1u : 0u, odd_q = 0;
             const int x0 = W > 1 ? (int)threadIdx.x : gl;
             for (int x = x0; 8 * x < tlen0; x += LANES) odd |= odd_codes(t[x], tlen0 - 8 * x);
             bool bad = odd & 1u;
@@ -181,12 +188,17 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
             }
             if (group_any(bad)) {
                 /* left to compare scoring: short pairs from the list's front, long ones from its end */
-                if (listed && gl == 0 && wi == 0) {
+                if (too_long()) {
+                    skip();
+                } else if (listed && gl == 0 && wi == 0) {
                     if (qlen0 >= PK_CMP_LONG) A.defer[A.n - 1 - (int)atomicAdd(A.ndefer + 1, 1u)] = (uint32_t)i;
                     else A.defer[atomicAdd(A.ndefer, 1u)] = (uint32_t)i;
                 }
                 has = false;
             }
+        } else if (too_long()) {
+            skip();
+            has = false;
         }
         const bool work = has && qlen0 > 0 && tlen0 > 0;
         const int qlen = work ? qlen0 : 0, tlen = work ? tlen0 : 0;
@@ -720,20 +732,22 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
         uint32_t *qu = A.queue + c;
         if constexpr (!FAST) { /* what the table-scoring launch left: long pairs, then short ones */
             if (k.group == 32)
-                pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l + (A.n - 1), (int)A.n_dev[1], qu, k.ring_cols, -1);
+                pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l + (A.n - 1), (int)A.n_dev[1], qu, k.ring_cols,
+                                                    k.max_q8, -1);
             else
-                pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols);
+                pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols, k.max_q8);
             continue;
         }
         switch (k.group) {
-        case 1: pk_pairs<1, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
-        case 2: pk_pairs<2, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
-        case 4: pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
-        case 8: pk_pairs<8, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
-        case 16: pk_pairs<16, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
-        case 32: pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols); break;
+        case 1: pk_pairs<1, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
+        case 2: pk_pairs<2, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
+        case 4: pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
+        case 8: pk_pairs<8, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
+        case 16: pk_pairs<16, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
+        case 32: pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l, nl, qu, k.ring_cols, k.max_q8); break;
         default:
-            if constexpr (W > 1) pk_pairs<32, W, ALGO, START, FAST>(A, P, tab, pk_smem, l, nl, qu, k.ring_cols);
+            if constexpr (W > 1)
+                pk_pairs<32, W, ALGO, START, FAST>(A, P, tab, pk_smem, l, nl, qu, k.ring_cols, k.max_q8);
             __syncthreads(); /* the block's rings become its warps' */
         }
     }

@@ -33,9 +33,10 @@ struct PkConst {
 constexpr int PK_FIFO = 32;
 
 /* One class of a launch: pairs list[first, first + n) on `group` lanes each
- * (32 * the block's warps: the block), with rings of ring_cols words. */
+ * (32 * the block's warps: the block), with rings of ring_cols words for
+ * queries of up to max_q8 bases (in whole words). */
 struct PkClass {
-    int32_t group, first, n, ring_cols;
+    int32_t group, first, n, ring_cols, max_q8;
 };
 constexpr int PK_CLASSES = 6;
 struct PkClasses {
@@ -64,9 +65,10 @@ struct PkLengths {
 /* the shapes of a batch's launches */
 struct PkPlan {
     int group[PK_CLASSES] = {};
-    int ring_cols[PK_CLASSES] = {};
+    int ring_cols[PK_CLASSES] = {}, max_q8[PK_CLASSES] = {};
     int warp_words = 0, warps = 0, blocks = 0;         /* blocks: most that are resident */
-    int cmp_cols[2] = {}, cmp_blocks = 0;              /* compare scoring: long pairs (32 lanes), short ones (4) */
+    /* compare scoring: long pairs (32 lanes), short ones (4) */
+    int cmp_cols[2] = {}, cmp_q8[2] = {}, cmp_blocks = 0;
 };
 
 /* The packed kernels take LOCAL, GLOBAL and target-tail SEMI_GLOBAL without a

@@ -73,7 +73,8 @@ struct Workspace {
     uint32_t *pk_defer = nullptr; /* pairs the packed table-scoring launches leave to the compare-scoring ones */
     size_t pk_defer_cap = 0;
     uint32_t *pk_q = nullptr;    /* PK_QUEUE_WORDS counters of the packed launches */
-    uint8_t *tb_kind = nullptr;  /* per pair of a traceback chunk: 1 = boundary checkpoints, 0 = direction tiles */
+    uint8_t *tb_kind = nullptr;  /* per pair of a traceback chunk: 1 = boundary checkpoints, 0 = direction tiles,
+                                    2 = not swept */
     size_t tb_kind_cap = 0;
     uint32_t *words = nullptr;   /* copies of packed words that CIGARs are written over */
     size_t words_cap = 0;

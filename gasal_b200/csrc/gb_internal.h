@@ -59,7 +59,8 @@ struct DpArgs {
                                            running maximum rose (ksw_extend2's max_off), or null */
     uint32_t *stuck;                    /* set when a bounded wait of a kernel ran out */
     uint8_t *tb_kind;                   /* per pair: 1 when its traceback storage holds boundary
-                                           checkpoints (dp_pk.cuh) instead of direction tiles */
+                                           checkpoints (dp_pk.cuh) instead of direction tiles, 2 when
+                                           it was not swept */
     uint32_t *defer, *ndefer;           /* warp-cooperative table-scoring launch: pairs it leaves to the
                                            compare-scoring launch, and their count */
 };
@@ -84,7 +85,7 @@ struct TbArgs {
     int32_t algo;
     Scores sc;
     int32_t head;                       /* SEMI_GLOBAL: which leading bases are free */
-    const uint8_t *kind;                /* per pair: 1 = checkpoints (traceback_points_kernel) */
+    const uint8_t *kind;                /* per pair: 1 = checkpoints (traceback_points_kernel), 2 = nothing to walk */
     const uint32_t *order;              /* visiting order of the checkpoint walks, or null */
     const uint32_t *pq, *pt, *t_off;    /* packed words, for recomputing blocks */
     int32_t c0, pa, pb;                 /* the packed kernels' offsets (PkConst) */

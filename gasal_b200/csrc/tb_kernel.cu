@@ -281,7 +281,7 @@ template <bool LOC> __global__ void __launch_bounds__(TBP_THREADS) traceback_poi
     bool have = slot < (shared_walk ? coop : a.n);
     if (have) {
         p = a.order ? (int)a.order[slot] : slot;
-        have = a.kind[p] != 0;
+        have = a.kind[p] == 1;
     }
     int qlen = 0, tlen = 0;
     if (have) qlen = (int)a.q_len[p], tlen = (int)a.t_len[p];
