@@ -25,7 +25,7 @@ N_CODE = 0x4E
 
 GB_OK = 0
 GB_STATUS = {0: "ok", -1: "bad argument", -2: "CUDA error", -3: "not ready", -4: "no work",
-             -5: "allocation failed", -6: "limit exceeded"}
+             -5: "allocation failed", -6: "limit exceeded", -7: "a wait inside a kernel ran out"}
 
 
 class GbParams(C.Structure):

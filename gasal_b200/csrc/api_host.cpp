@@ -1123,6 +1123,8 @@ void graph_stats(int64_t out[4])
     for (int k = 0; k < 4; k++) out[k] = g_graph_stats[k].load();
 }
 
+bool took_stuck(gasal_gpu_storage_t *s) { return gb::take_stuck(state_of(s).ws); }
+
 int is_done(gasal_gpu_storage_t *s, bool fatal)
 {
     if (s->is_free == 1) return -2;
@@ -1137,6 +1139,10 @@ int is_done(gasal_gpu_storage_t *s, bool fatal)
     gasal_host_batch_reset(s);
     s->is_free = 1;
     s->current_n_alns = 0;
+    if (took_stuck(s)) {
+        if (fatal) exit(EXIT_FAILURE);
+        return GB_ERR_WAIT;
+    }
     return 0;
 }
 

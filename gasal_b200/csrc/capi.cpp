@@ -18,6 +18,7 @@ namespace gbapi {
 int aln_async(gasal_gpu_storage_t *s, uint32_t qbytes, uint32_t tbytes, uint32_t n, Parameters *params, bool fatal,
               int zdrop);
 int is_done(gasal_gpu_storage_t *s, bool fatal);
+bool took_stuck(gasal_gpu_storage_t *s);
 void graph_stats(int64_t out[4]);
 }
 
@@ -248,7 +249,7 @@ int gb_align(const gb_params_t *p, const gb_batch_t *b, gb_out_t *o)
     int rc = gbapi::aln_async(s, b->q_bytes, b->t_bytes, n, &params, false, p->zdrop);
     if (rc == GB_OK) {
         cudaError_t e = cudaStreamSynchronize(s->str);
-        rc = e == cudaSuccess ? GB_OK : GB_ERR_CUDA;
+        rc = e != cudaSuccess ? GB_ERR_CUDA : gbapi::took_stuck(s) ? GB_ERR_WAIT : GB_OK;
     }
     if (rc == GB_OK) {
         gasal_res_t *r = s->host_res;
@@ -330,17 +331,20 @@ void dev_args(const gb_params_t *p, const gb_dev_batch_t *b, const gb_dev_out_t 
 extern "C" int gb_release_workspaces(void)
 {
     if (cudaDeviceSynchronize() != cudaSuccess) return GB_ERR_CUDA;
+    bool stuck = false;
     {
         std::lock_guard<std::mutex> lk(g_dev_mu);
         for (auto &kv : g_dev_ws) {
+            stuck |= gb::take_stuck(kv.second->ws);
             gb::release_workspace(kv.second->ws);
             delete kv.second;
         }
         g_dev_ws.clear();
     }
-    gb::mix_release_all();
+    stuck |= gb::mix_release_all();
     gb::band_release_all();
-    return cudaGetLastError() == cudaSuccess ? GB_OK : GB_ERR_CUDA;
+    if (cudaGetLastError() != cudaSuccess) return GB_ERR_CUDA;
+    return stuck ? GB_ERR_WAIT : GB_OK;
 }
 
 extern "C" int gb_align_dev(const gb_params_t *p, const gb_dev_batch_t *b, const gb_dev_out_t *o, void *stream)

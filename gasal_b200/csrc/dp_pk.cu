@@ -237,7 +237,7 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     /* the table-scoring launch, then the compare-scoring one over the pairs it
      * left (a target with another code than A, C, G, T, N) */
     DpArgs f = a;
-    f.queue = wq, f.defer = defer, f.ndefer = wq + PK_CLASSES + 2, f.n_dev = nullptr, f.stuck = wq + PK_CLASSES + 4;
+    f.queue = wq, f.defer = defer, f.ndefer = wq + PK_CLASSES + 2, f.n_dev = nullptr;
     cudaError_t e = launch(p.warps == 4 ? PK_W4 : p.warps == 2 ? PK_W2 : PK_W1, f, cl, list,
                            (int)std::min<long>((warps + p.warps - 1) / p.warps, p.blocks), p.warps);
     if (e != cudaSuccess) return e;

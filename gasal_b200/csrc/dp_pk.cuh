@@ -35,8 +35,10 @@
  * the rest of the launch.  Warp x takes the bands of every W-th round; the warps run
  * unsynchronised, each
  * handing its last virtual lane's outputs to the next through a fifo of
- * PK_FIFO words with counters (bounded waits), the last to the first through
- * the ring.  No warp waits in a circle: a round has at least as many steps as
+ * PK_FIFO words with counters, the last to the first through the ring.  The
+ * waits are bounded: one that runs out ends the warp's sweep (one lane polls, so
+ * the whole warp leaves at the same poll) and sets a word that the host reports
+ * as an error.  No warp waits in a circle: a round has at least as many steps as
  * the group virtual lanes, and the ring holds a whole one, so the last warp
  * never waits for room.
  *
@@ -65,7 +67,6 @@ namespace gb {
 namespace {
 
 constexpr uint32_t PAD_WORD = 0xEEEEEEEEu; /* eight N codes */
-constexpr int PK_SPINS = 1 << 22;          /* bound of a wait on another warp of the group */
 
 __device__ __forceinline__ int half_of(uint32_t x, bool hi) { return (int)(int16_t)(hi ? x >> 16 : x & 0xFFFFu); }
 /* both halves of x with half `hi` replaced by v (16 bits) */
@@ -142,6 +143,12 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
      * pass's first band with a hit; the group's item and results */
     __shared__ volatile int prod[W], cons[W], s_stop;
     __shared__ int s_item, s_key[W], s_res[3];
+    auto ran_out = [&]() {
+        if (lane == 0) {
+            *const_cast<volatile uint32_t *>(A.stuck) = 1u;
+            __threadfence_system();
+        }
+    };
     auto group_any = [&](bool x) -> bool {
         if (W > 1) return __syncthreads_or(x);
         return __ballot_sync(0xFFFFFFFFu, x) & gmask;
@@ -299,10 +306,9 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
                 if (W > 1 && s < rounds * per) { /* wait for the word that lane 0 reads */
                     const int src = wi > 0 ? wi - 1 : W - 1, need = wi > 0 ? s : s - per;
                     for (int spin = 0; need >= avail;) {
-                        avail = prod[src];
-                        if (need < 0) break;
-                        if (++spin > PK_SPINS) {
-                            *A.stuck = 1u; /* never: the producer's step does not wait on this one */
+                        avail = __shfl_sync(0xFFFFFFFFu, prod[src], 0);
+                        if (need >= avail && ++spin > A.spins) {
+                            ran_out(); /* never: the producer's step does not wait on this one */
                             wend = s;
                             break;
                         }
@@ -487,14 +493,13 @@ __device__ __forceinline__ void pk_pairs(const DpArgs &A, const PkConst &P, cons
                     if (x >= 0 && x < wanted && on) {
                         if (wi < W - 1) {
                             for (int spin = 0; taken + PK_FIFO <= x;) { /* room in the fifo */
-                                taken = cons[wi + 1];
-                                if (++spin > PK_SPINS) {
-                                    *A.stuck = 1u;
+                                taken = __shfl_sync(0xFFFFFFFFu, cons[wi + 1], G - 1);
+                                if (taken + PK_FIFO <= x && ++spin > A.spins) {
+                                    ran_out();
                                     wend = s;
                                     break;
                                 }
                             }
-                            __syncwarp();
                         }
                         if (gl == G - 1) {
                             uint4 *rp = reinterpret_cast<uint4 *>(

@@ -82,7 +82,7 @@ PkConst pk_const(int algo, const Scores &sc);
 bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPlan &p);
 /* n[c]: the pairs of class c, in list order.  wq: PK_QUEUE_WORDS zeroed words;
  * defer: a word per pair */
-constexpr int PK_QUEUE_WORDS = PK_CLASSES + 5;
+constexpr int PK_QUEUE_WORDS = PK_CLASSES + 4;
 cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc, const PkPlan &p, const uint32_t *list,
                          const int *n, uint32_t *defer, uint32_t *wq, cudaStream_t s);
 

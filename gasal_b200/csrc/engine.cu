@@ -52,6 +52,7 @@ Settings &settings()
         if (const char *e = getenv("GASAL_B200_MIN_ORDER_PAIRS")) v.min_order_pairs = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_MIN_QREGS")) v.wc_min_qregs = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_BIG_GROUP")) v.wc_big_group = atoi(e);
+        if (const char *e = getenv("GASAL_B200_WAIT_SPINS")) v.wait_spins = atoi(e);
         if (const char *e = getenv("GASAL_B200_KSW_GROUPS")) v.ksw_groups = atoi(e);
         return v;
     }();
@@ -138,6 +139,16 @@ Workspace::~Workspace()
      * context is current; nothing to do at static destruction time */
 }
 
+bool take_stuck(Workspace &w)
+{
+    volatile uint32_t *word = w.stuck;
+    if (!word || *word == 0) return false;
+    *word = 0;
+    fprintf(stderr, "[GASAL-B200 ERROR] a wait between the warps of a packed sweep ran out; an earlier batch's results "
+                    "are not right\n");
+    return true;
+}
+
 void release_workspace(Workspace &w)
 {
     if (w.tb) cudaFree(w.tb);
@@ -153,6 +164,7 @@ void release_workspace(Workspace &w)
     if (w.pk_q) cudaFree(w.pk_q);
     if (w.tb_kind) cudaFree(w.tb_kind);
     if (w.words) cudaFree(w.words);
+    if (w.stuck) cudaFreeHost(w.stuck);
     if (w.aux) cudaStreamDestroy(w.aux);
     if (w.queue) cudaFree(w.queue);
     if (w.fork) cudaEventDestroy(w.fork);
@@ -308,6 +320,16 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
         cudaGetLastError();
         return GB_ERR_ALLOC;
     }
+    /* several warps to a pair: they wait for one another */
+    const bool waits = std::any_of(p.pkp.group, p.pkp.group + PK_CLASSES, [](int g) { return g > 32; });
+    if (waits && !ws.stuck) {
+        if (cudaHostAlloc((void **)&ws.stuck, sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            ws.stuck = nullptr;
+            return GB_ERR_ALLOC;
+        }
+        *ws.stuck = 0;
+    }
     p.pkc = pk_const(cfg.algo, cfg.sc);
     p.order_on = order;
     p.pk = true;
@@ -454,6 +476,7 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
     a.score = o.score, a.q_end = o.q_end, a.t_end = o.t_end, a.q_start = o.q_start, a.t_start = o.t_start;
     a.score2 = o.score2, a.q_end2 = o.q_end2, a.t_end2 = o.t_end2;
     a.max_off = cfg.algo == KSW_ ? o.max_off : nullptr;
+    a.stuck = ws.stuck, a.spins = st.wait_spins;
     a.sc = cfg.sc, a.head = cfg.head, a.tail = cfg.tail, a.k_band = cfg.k_band, a.zdrop = cfg.zdrop, a.mql = cfg.mql;
     if (!ws.queue && dev_malloc((void **)&ws.queue, 128) != cudaSuccess) {
         cudaGetLastError();
@@ -648,6 +671,7 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
 int plan_batch(const RunCfg &cfg, const DevBatch &b, const DevOut &o, Workspace &ws, Plan &p, cudaStream_t s)
 {
     if (b.n <= 0) return GB_ERR_ARG;
+    if (take_stuck(ws)) return GB_ERR_WAIT; /* the caller learns of it here at the latest */
     return plan_batch_with(true, cfg, b, o, ws, p, s);
 }
 

@@ -73,6 +73,7 @@ struct Workspace {
     uint32_t *pk_defer = nullptr; /* pairs the packed table-scoring launches leave to the compare-scoring ones */
     size_t pk_defer_cap = 0;
     uint32_t *pk_q = nullptr;    /* PK_QUEUE_WORDS counters of the packed launches */
+    uint32_t *stuck = nullptr;   /* pinned: set by a kernel whose bounded wait ran out (take_stuck) */
     uint8_t *tb_kind = nullptr;  /* per pair of a traceback chunk: 1 = boundary checkpoints, 0 = direction tiles,
                                     2 = not swept */
     size_t tb_kind_cap = 0;
@@ -99,8 +100,12 @@ struct Workspace {
 /* Frees every buffer, stream and event of a workspace (no work of it may be
  * in flight) and leaves it empty, ready to grow again. */
 void release_workspace(Workspace &w);
-/* the buffers gb_align_dev_mixed keeps per (device, stream) (mixed.cu) */
-void mix_release_all();
+/* whether a wait of an earlier batch on this workspace ran out (its results are
+ * not right): says so on stderr and clears the word */
+bool take_stuck(Workspace &w);
+/* the buffers gb_align_dev_mixed keeps per (device, stream) (mixed.cu); true
+ * when a kind's workspace had its word set */
+bool mix_release_all();
 /* the band entry points' per-stream workspaces (band_api.cu) */
 void band_release_all();
 
@@ -190,6 +195,7 @@ struct Settings {
     const void *band_model = nullptr; /* installed band MLP (BF16 parameters on the device) */
     int band_min = 16, band_max = 1024;
     int wc_big_group = 0;       /* lane group of the 127+ word launch: 0 = automatic (64 when it fits), 32 or 64 */
+    int wait_spins = 1 << 22;   /* polls of a wait between warps before it gives up (0.2 s or so) */
     int ksw_groups = 1;         /* unbanded ksw pairs of at most 31 query words run 4 to a warp (lane groups) */
 };
 Settings &settings();

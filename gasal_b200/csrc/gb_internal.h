@@ -57,7 +57,8 @@ struct DpArgs {
                                            one slot of scratch_cols words per lane group of the grid */
     int32_t *max_off;                   /* unbanded ksw: largest |column - row| of the cells where the
                                            running maximum rose (ksw_extend2's max_off), or null */
-    uint32_t *stuck;                    /* set when a bounded wait of a kernel ran out */
+    uint32_t *stuck;                    /* host-mapped word, set when a bounded wait of a kernel ran out */
+    int32_t spins;                      /* polls that such a wait makes at most */
     uint8_t *tb_kind;                   /* per pair: 1 when its traceback storage holds boundary
                                            checkpoints (dp_pk.cuh) instead of direction tiles, 2 when
                                            it was not swept */

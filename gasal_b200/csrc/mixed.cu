@@ -98,15 +98,20 @@ std::unordered_map<unsigned long long, MixState *> g_mix;
 } // namespace
 
 /* every stream's mixed-dispatch buffers and kind workspaces (gb_release_workspaces) */
-void mix_release_all()
+bool mix_release_all()
 {
     std::lock_guard<std::mutex> lk(g_mix_mu);
+    bool stuck = false;
     for (auto &kv : g_mix) {
         MixState *m = kv.second;
-        for (auto &w : m->ws) release_workspace(w);
+        for (auto &w : m->ws) {
+            stuck |= take_stuck(w);
+            release_workspace(w);
+        }
         delete m;
     }
     g_mix.clear();
+    return stuck;
 }
 
 namespace {
@@ -204,6 +209,9 @@ extern "C" int gb_align_dev_mixed(const gb_params_t *kinds, int n_kinds, const u
     MixState *mp = mix_state(s);
     if (!mp) return GB_ERR_CUDA;
     MixState &m = *mp;
+    bool stuck = false;
+    for (auto &w : m.ws) stuck |= take_stuck(w);
+    if (stuck) return GB_ERR_WAIT; /* before anything of this call is queued */
     if ((rc = mix_streams(m)) != GB_OK) return rc;
     const size_t n = (size_t)b->n;
     if ((rc = mix_reserve(m, n)) != GB_OK) return rc;

@@ -30,7 +30,8 @@ enum gb_status {
     GB_ERR_NOT_READY = -3, /* work still in flight */
     GB_ERR_NO_WORK = -4,   /* nothing was launched on this stream */
     GB_ERR_ALLOC = -5,     /* device or pinned allocation failed */
-    GB_ERR_LIMIT = -6      /* a size is beyond a documented limit */
+    GB_ERR_LIMIT = -6,     /* a size is beyond a documented limit */
+    GB_ERR_WAIT = -7       /* a wait inside a kernel ran out: that batch's results are not right */
 };
 
 /* ---- per-launch options: the fields of GASAL2's Parameters that the
@@ -163,7 +164,7 @@ int gasal_c_set_device(int gpu);
 
 /* gasal_aln_async / gasal_is_aln_async_done, reference
  * src/gasal_align.h:116-120.  aln_async returns a gb_status; is_done returns
- * 0 (done), -1 (running), -2 (nothing launched) or GB_ERR_CUDA. */
+ * 0 (done), -1 (running), -2 (nothing launched), GB_ERR_CUDA or GB_ERR_WAIT. */
 int gasal_c_aln_async(void *storage, uint32_t query_batch_bytes, uint32_t target_batch_bytes, uint32_t n_alns,
                       void *params);
 int gasal_c_is_aln_async_done(void *storage);
@@ -178,7 +179,11 @@ int gb_align(const gb_params_t *p, const gb_batch_t *b, gb_out_t *o);
  * (a cudaStream_t, NULL = legacy default stream).  Uses a workspace per
  * (device, stream) that the library grows on demand; calls on one stream must
  * come from one host thread at a time.  The device half of gasal_aln_async
- * (src/gasal_align.cu:180-264).  n == 0 returns GB_OK and launches nothing. */
+ * (src/gasal_align.cu:180-264).  n == 0 returns GB_OK and launches nothing.
+ * Kernels whose warps wait for one another give up after a bounded number of
+ * polls; should that happen, the batch's results are not right, and the next
+ * call on the stream (or gb_release_workspaces) returns GB_ERR_WAIT.  The
+ * storage calls report it from gasal_is_aln_async_done, gb_align itself. */
 int gb_align_dev(const gb_params_t *p, const gb_dev_batch_t *b, const gb_dev_out_t *o, void *stream);
 
 /* The two preparation kernels alone, on device buffers, queued on `stream`:
