@@ -365,8 +365,10 @@ extern "C" int gb_align_dev(const gb_params_t *p, const gb_dev_batch_t *b, const
  * events on `stream`, `reps` runs after one warm-up run each) and keeps the
  * fastest.  Candidates: DP block 32/64/128 x warp-cooperative threshold
  * 16/32/48/64 query words x lane groups automatic/8/16/32 (LOCAL, GLOBAL and
- * target-tail SEMI_GLOBAL; other algorithms keep the
- * current threshold). */
+ * target-tail SEMI_GLOBAL; other algorithms keep the current threshold).  The
+ * packed kernels read none of these: a batch that they take whole is timed
+ * under the current settings alone, and one whose 127+ word pairs run
+ * warp-cooperative beside them under each lane group. */
 namespace {
 thread_local char g_last_error[256] = "";
 void set_last_error(const char *where, cudaError_t e)
@@ -410,10 +412,16 @@ extern "C" int gb_autotune(const gb_params_t *p, const gb_dev_batch_t *b, const 
     gb::Settings &st = gb::settings();
     const gb::Settings saved = st;
     const cudaStream_t s = (cudaStream_t)stream;
+    gb::Plan route;
+    int rc = gb::plan_batch(cfg, db, dout, w->ws, route, s);
+    if (rc != GB_OK) return rc;
     std::vector<int> blocks = {32, 64, 128};
     std::vector<int> wcs = {st.wc_min_qregs};
     std::vector<int> groups = {st.wc_group};
-    if (p->algo == LOCAL || p->algo == GLOBAL || (p->algo == SEMI_GLOBAL && p->tail == TARGET)) {
+    if (route.pk) {
+        blocks = {st.block};
+        if (route.pk_wc) groups = {0, 8, 16, 32};
+    } else if (p->algo == LOCAL || p->algo == GLOBAL || (p->algo == SEMI_GLOBAL && p->tail == TARGET)) {
         wcs = {16, 32, 48, 64};
         groups = {0, 8, 16, 32};
     }
@@ -423,7 +431,6 @@ extern "C" int gb_autotune(const gb_params_t *p, const gb_dev_batch_t *b, const 
         cudaEventDestroy(e0);
         return GB_ERR_CUDA;
     }
-    int rc = GB_OK;
     float best_t = 0.f;
     gb_tuning_t bt{saved.block, saved.wc_min_qregs, saved.min_order_pairs, saved.ksw_wc, saved.split_start,
                    saved.persistent, saved.wc_group};

@@ -146,6 +146,7 @@ bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPl
         if (cl[c].n) n += cl[c].n, max_q = std::max(max_q, cl[c].max_q);
     double best_t = 0;
     for (int w : {1, 2, 4}) {
+        if (forced > 32 && 32 * w != forced) continue;
         const KernelUse u = kernel_use(algo, w == 4 ? PK_W4 : w == 2 ? PK_W2 : PK_W1, start);
         const double hand = w == 4 ? 1.45 : 1.15;
         double cost[PK_CLASSES][WIDE + 1], longest[PK_CLASSES][WIDE + 1], limits[PK_CLASSES * (WIDE + 1)];

@@ -78,7 +78,8 @@ struct PkPlan {
 bool pk_scores_ok(int algo, const Scores &sc);
 bool pk_fits(int algo, const Scores &sc, uint32_t max_q, uint32_t max_t, uint32_t max_min);
 PkConst pk_const(int algo, const Scores &sc);
-/* false: no shape fits.  forced: lanes per pair (8, 16, 32, 64), 0 = by the model */
+/* false: no shape fits.  forced: least lanes per pair (1 to 32), or the 64 or
+ * 128 of a two- or four-warp block; 0 = by the model */
 bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPlan &p);
 /* n[c]: the pairs of class c, in list order.  wq: PK_QUEUE_WORDS zeroed words;
  * defer: a word per pair */

@@ -51,6 +51,7 @@ Settings &settings()
         if (const char *e = getenv("GASAL_B200_BLOCK")) v.block = atoi(e);
         if (const char *e = getenv("GASAL_B200_MIN_ORDER_PAIRS")) v.min_order_pairs = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_MIN_QREGS")) v.wc_min_qregs = atoi(e);
+        if (const char *e = getenv("GASAL_B200_PK_GROUP")) v.pk_group = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_BIG_GROUP")) v.wc_big_group = atoi(e);
         if (const char *e = getenv("GASAL_B200_WAIT_SPINS")) v.wait_spins = atoi(e);
         if (const char *e = getenv("GASAL_B200_KSW_GROUPS")) v.ksw_groups = atoi(e);
@@ -313,8 +314,7 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
         }
     }
     const int start = cfg.algo == GLOBAL_ && cfg.start == WITH_START_ ? WITHOUT_START_ : cfg.start;
-    const int forced = st.wc_group;
-    if (!pk_plan(cfg.algo, start, cl, sms, forced, p.pkp)) return GB_OK;
+    if (!pk_plan(cfg.algo, start, cl, sms, st.pk_group, p.pkp)) return GB_OK;
     if (grow((void **)&ws.pk_defer, &ws.pk_defer_cap, (size_t)b.n, 4) != GB_OK) return GB_ERR_ALLOC;
     if (!ws.pk_q && dev_malloc((void **)&ws.pk_q, PK_QUEUE_WORDS * 4) != cudaSuccess) {
         cudaGetLastError();

@@ -194,6 +194,8 @@ struct Settings {
                                    pair on a grid over the batch */
     const void *band_model = nullptr; /* installed band MLP (BF16 parameters on the device) */
     int band_min = 16, band_max = 1024;
+    int pk_group = 0;           /* packed kernels: least lanes per pair (a power of two up to 32), 64 or 128 (the
+                                   warps of a two- or four-warp block), or 0 to pick by the model (pk_plan) */
     int wc_big_group = 0;       /* lane group of the 127+ word launch: 0 = automatic (64 when it fits), 32 or 64 */
     int wait_spins = 1 << 22;   /* polls of a wait between warps before it gives up (0.2 s or so) */
     int ksw_groups = 1;         /* unbanded ksw pairs of at most 31 query words run 4 to a warp (lane groups) */

@@ -282,7 +282,11 @@ int gb_graph_stats(int64_t *counts);
  * (LOCAL/GLOBAL/target-tail SEMI_GLOBAL; at least 8, never fewer than
  * wc_group, which that kernel needs, and more than 127 count as 127);
  * min_order_pairs: batches with at least this many pairs are
- * visited length-binned.  Results never depend on these. */
+ * visited length-binned (by the packed kernels also batches of more than 64
+ * whose longest query is over 1.5 times the shortest, unless it is above
+ * 2^29).  The packed kernels -- LOCAL, GLOBAL and target-tail SEMI_GLOBAL
+ * without a second best, values within 15 bits -- take no other of these but
+ * persistent.  Results never depend on these. */
 typedef struct {
     int32_t block;
     int32_t wc_min_qregs;
@@ -291,8 +295,8 @@ typedef struct {
     int32_t split_start;   /* 1: LOCAL / SEMI_GLOBAL start passes run as their own launch, pairs re-ordered
                               by forward score (default); 0: in the forward launch */
     int32_t persistent;    /* 1: one-pair-per-thread launches are persistent, warps pulling pairs from a
-                              device counter (default); 0: one thread per pair on a grid over the batch.
-                              With min_order_pairs above the batch size, ksw_warp 0 and split_start 0
+                              device counter (default); 0: one thread per pair on a grid over the batch,
+                              and no packed kernels.  With min_order_pairs above the batch size, ksw_warp 0 and split_start 0
                               this is the plain full-DP form: every pair one per thread, in input order */
     int32_t wc_group;      /* lanes per pair in the warp-cooperative kernels: 64 (two warps per pair),
                               32, 16 or 8 (a warp sweeps 32/wc_group pairs side by side), or 0 (default):
@@ -304,9 +308,11 @@ int gb_set_tuning(const gb_tuning_t *t);
 int gb_get_tuning(gb_tuning_t *t);
 
 /* Autotuner (no reference counterpart): runs gb_align_dev on the caller's
- * batch under each candidate tuning (block 32/64/128; for LOCAL, GLOBAL and
- * target-tail SEMI_GLOBAL also warp-cooperative thresholds 16/32/48/64 words
- * x lane groups automatic/8/16/32, thresholds below the group skipped), `reps` timed runs each
+ * batch under each candidate tuning that its kernels read (block 32/64/128;
+ * for LOCAL, GLOBAL and target-tail SEMI_GLOBAL also warp-cooperative
+ * thresholds 16/32/48/64 words x lane groups automatic/8/16/32, thresholds
+ * below the group skipped; for a batch of the packed kernels the current
+ * settings alone, or each lane group for its pairs beyond 15 bits), `reps` timed runs each
  * after a warm-up run, timed with CUDA events on `stream`; installs and
  * returns the fastest (best_ms: its mean milliseconds per run; may be NULL).
  * The outputs hold the batch's results afterwards.  Synchronizes `stream`;

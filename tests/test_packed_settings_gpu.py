@@ -1,0 +1,98 @@
+"""Settings around the packed kernels: every lane group that can be forced gives
+the oracle's results, the warp-cooperative kernels' lane group leaves packed
+batches alone, and the autotuner tries only what the batch's route uses."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from gasal_b200 import lib as gl
+from gasal_b200 import workloads as W
+from gasal_b200.capi import Batch, Params, LOCAL, SEMI_GLOBAL, WITH_START, TARGET
+from oracle.bindings import oracle_align
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SEMI = Params(algo=SEMI_GLOBAL, start_pos=WITH_START, head=TARGET, tail=TARGET)
+
+
+def _device(torch, p, b):
+    dev = torch.device("cuda", 0)
+
+    def up(a, dt=None):
+        return torch.from_numpy(np.ascontiguousarray(a).view(dt or a.dtype)).to(dev)
+    keep = {"q": up(b.q), "t": up(b.t), "pq": torch.zeros(b.q.shape[0] // 8, dtype=torch.int32, device=dev),
+            "pt": torch.zeros(b.t.shape[0] // 8, dtype=torch.int32, device=dev)}
+    for k in ("q_off", "t_off", "q_len", "t_len"):
+        keep[k] = up(getattr(b, k), np.int32)
+    outs = {k: torch.zeros(b.n, dtype=torch.int32, device=dev) for k in ("score", "q_end", "t_end", "q_start", "t_start")}
+    m = {"q_bytes": b.q.shape[0], "t_bytes": b.t.shape[0]}
+    m.update({k: v.data_ptr() for k, v in keep.items()})
+    m.update({"out_" + k: v.data_ptr() for k, v in outs.items()})
+    return m, keep, outs
+
+
+FORCED = """
+import os, sys
+sys.path[:0] = [sys.argv[1], os.path.join(sys.argv[1], "tests")]
+import test_packed_gpu as T
+for p in T.MODES:
+    T.test_edges_of_words_bands_and_rounds(p, 0)
+    T.test_few_long_pairs(p, 9)
+    T.test_mixed_lengths_in_order(p)
+"""
+
+
+@pytest.mark.parametrize("group", [1, 2, 4, 8, 16, 32, 64, 128])
+def test_forced_lane_groups(group):
+    """The edge shapes, a few long pairs and the ordered mix of the packed
+    kernels' tests on at least `group` lanes per pair."""
+    r = subprocess.run([sys.executable, "-c", FORCED, ROOT], env=dict(os.environ, GASAL_B200_PK_GROUP=str(group)),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_warp_cooperative_group_leaves_short_reads_alone():
+    """100,000 short reads take the same time with any wc_group (while it
+    forced the packed kernels' lanes too, 32 cost them six times as much)."""
+    torch = pytest.importorskip("torch")
+    b = W.workload0(100000, seed=5)
+    m, keep, outs = _device(torch, SEMI, b)
+    s = torch.cuda.current_stream().cuda_stream
+    ms = {}
+    saved = gl.get_tuning()
+    try:
+        for g in (0, 32):
+            gl.set_tuning(wc_group=g)
+            for _ in range(3):
+                gl.align_dev(SEMI, m, b.q_len, b.t_len, s)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(10):
+                gl.align_dev(SEMI, m, b.q_len, b.t_len, s)
+            e1.record()
+            torch.cuda.synchronize()
+            ms[g] = e0.elapsed_time(e1)
+    finally:
+        gl.set_tuning(**saved)
+    assert ms[32] < 2 * ms[0], ms
+
+
+def test_autotune_of_a_packed_batch_keeps_the_settings():
+    torch = pytest.importorskip("torch")
+    p = Params(algo=LOCAL, start_pos=WITH_START)
+    b = W.workload2(3000, seed=6)
+    m, keep, outs = _device(torch, p, b)
+    saved = gl.get_tuning()
+    try:
+        best = gl.autotune(p, m, b.q_len, b.t_len, torch.cuda.current_stream().cuda_stream, reps=1)
+        torch.cuda.synchronize()
+        assert best["ms"] > 0
+        assert gl.get_tuning() == saved
+        for k, v in oracle_align(p, b).as_dict(p).items():
+            assert np.array_equal(outs[k].cpu().numpy(), v), k
+    finally:
+        gl.set_tuning(**saved)
