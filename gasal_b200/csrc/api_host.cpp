@@ -278,7 +278,7 @@ void batch_signature(std::vector<uint8_t> &v, const gasal_gpu_storage_t *s, cons
     put(v, plan.mt8_big), put(v, (const void *)ss.ws.wc_rows);
     put(v, (const void *)cfg.band_w), put(v, cfg.band_model), put(v, cfg.band_min), put(v, cfg.band_max);
     put(v, (const void *)cfg.band_ok);
-    put(v, plan.pk), put(v, plan.pk_wc), put(v, plan.pk_all), put(v, plan.pkc), put(v, plan.pkp);
+    put(v, plan.pk), put(v, plan.pk_wc), put(v, plan.pkc), put(v, plan.pkp); /* (pk_n holds the classes launched) */
     const void *pk_ptrs[] = {ss.ws.pk_defer, ss.ws.pk_q, ss.ws.tb_kind, ss.ws.words};
     for (const void *q : pk_ptrs) put(v, q);
     for (int c : plan.pk_n) put(v, c);

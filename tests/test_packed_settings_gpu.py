@@ -1,6 +1,8 @@
 """Settings around the packed kernels: every lane group that can be forced gives
 the oracle's results, the warp-cooperative kernels' lane group leaves packed
-batches alone, and the autotuner tries only what the batch's route uses."""
+batches alone, the autotuner tries only what the batch's route uses, and a
+storage's graph is replayed for batches that differ in nothing the launches
+depend on."""
 import os
 import subprocess
 import sys
@@ -96,3 +98,29 @@ def test_autotune_of_a_packed_batch_keeps_the_settings():
             assert np.array_equal(outs[k].cpu().numpy(), v), k
     finally:
         gl.set_tuning(**saved)
+
+def test_graph_replayed_for_an_unordered_batch_of_other_lengths():
+    """Fewer pairs than the length order takes, of nearly equal lengths: one
+    launch whatever their classes, so the same bytes and pairs replay the
+    graph."""
+    rng = np.random.default_rng(7)
+    p = Params(algo=LOCAL, start_pos=WITH_START)
+
+    def batch(lens):
+        q = [rng.choice(np.frombuffer(b"ACGT", np.uint8), n).tobytes() for n in lens]
+        return Batch.from_seqs(q, [(x + b"ACGTTGCA" * 20)[:160] for x in q])
+    a, b = batch([120] * 50 + [128] * 50), batch([112] + [120] * 48 + [128] * 51)
+    assert a.q.shape == b.q.shape and a.t.shape == b.t.shape
+    gl.set_graphs(True)
+    with gl.Streams(1, 160, 160, 100, p) as st:
+        seen = []
+        for x in (a, b):
+            s0 = gl.graph_stats()
+            qi, ti = st.fill_fast(0, x)
+            st.aln_async(0, qi, ti, x.n)
+            st.wait(0)
+            got = st.results(0, x.n, x)
+            for k, v in oracle_align(p, x).as_dict(p).items():
+                assert np.array_equal(got[k], v), k
+            seen.append({k: v - s0[k] for k, v in gl.graph_stats().items()})
+    assert seen[0]["instantiated"] == 1 and seen[1]["relaunched"] == 1, seen
