@@ -51,6 +51,7 @@ Settings &settings()
         if (const char *e = getenv("GASAL_B200_BLOCK")) v.block = atoi(e);
         if (const char *e = getenv("GASAL_B200_MIN_ORDER_PAIRS")) v.min_order_pairs = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_MIN_QREGS")) v.wc_min_qregs = atoi(e);
+        if (const char *e = getenv("GASAL_B200_TB_COOP")) v.tb_coop = atoi(e);
         if (const char *e = getenv("GASAL_B200_PK_GROUP")) v.pk_group = atoi(e);
         if (const char *e = getenv("GASAL_B200_WC_BIG_GROUP")) v.wc_big_group = atoi(e);
         if (const char *e = getenv("GASAL_B200_WAIT_SPINS")) v.wait_spins = atoi(e);
@@ -287,7 +288,13 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
         }
     }
     for (int c = 0; c < PK_CLASSES; c++) p.pk_all[c] = cl[c].n;
-    /* an unordered batch is one class: equal lengths, or too few pairs for the order to matter */
+    /* An unordered batch is one class: equal lengths, or too few pairs for the order to matter.
+     * Queries only are compared (the bound on a pair's lanes is its query; targets of any length
+     * share a class).  The order's three launches cost 20 us; without it every pair has the lane
+     * group and ring of the longest.  LOCAL of 50-1,000 bp, us a call ordered / not: 100 pairs
+     * 644 / 626, 300 655 / 655, 1,000 664 / 904, 2,000 943 / 1,736; of 50-5,000 bp, 100 pairs
+     * 1,994 / 1,687, 1,000 1,712 / 3,195; GLOBAL of 50-1,000 bp, 100 pairs 256 / 225, 1,000
+     * 306 / 323: the lines meet at about 300 pairs. */
     const bool order = b.n >= st.min_order_pairs || (b.n > 64 && st.min_order_pairs <= (1 << 29) && max_q > min_q + min_q / 2);
     if (!order) {
         PkLengths &z = cl[0];
@@ -925,10 +932,15 @@ static int enqueue_align(const RunCfg &cfg, const DevBatch &b, const DevOut &o, 
             t.pq = ca.pq, t.pt = ca.pt, t.t_off = ca.t_off;
             t.c0 = p.pkc.c0, t.pa = p.pkc.a, t.pb = p.pkc.b;
             /* 8 lanes to the pairs whose walks would outlast the rest: queries of 127+ words,
-             * and the longest of any batch while its threads leave the GPU idle */
+             * and the longest tb_coop pairs of any batch while its threads leave the GPU idle.
+             * Measured on a B200, us a call with none / 2,048 / 8,192 / 32,768 pairs on 8 lanes:
+             * 100k LOCAL of 50-5,000 bp 16,790 / 13,320 / 13,370 / 13,630; LOCAL of 50-1,000 bp, 1k
+             * pairs 1,814 / 1,151 / 1,150 / 1,154, 8k 2,514 / 1,844 / 1,843 / 1,846, 32k 4,262 /
+             * 3,965 / 3,710 / 3,792; 100k GLOBAL of those lengths 5,961 / 5,890 / 6,387 / 7,094 (the
+             * one batch that 2,048 suits better); 8k GLOBAL of 150 bp 429 / 422 / 374 / 376 */
             const int *pn = p.pk_n.data() + PK_CLASSES * c;
-            const int longest = p.order_on ? pn[0] + pn[1] : 0;
-            GB_CUDA(launch_traceback_points(t, std::max(longest, TB_COOP_PAIRS), s));
+            const int longest = p.order_on ? pn[0] + pn[1] : 0, coop = settings().tb_coop;
+            GB_CUDA(launch_traceback_points(t, coop < 0 ? 0 : std::max(longest, coop), s));
         }
         if (!p.pk || p.pk_wc) GB_CUDA(launch_traceback(t, s));
         timing_mark(K_TB, false, s);

@@ -114,7 +114,6 @@ void band_release_all();
  * of DP size (2,560 x 2,560 bases), whose sweeps would outlast the rest of a
  * launch; class c > 0 the other queries of at least PK_CLASS_WORDS[c] words
  * (and fewer than class c-1's). */
-constexpr int TB_COOP_PAIRS = 8192;
 constexpr uint32_t PK_LONG_UNITS = 25;
 constexpr uint32_t PK_CLASS_WORDS[PK_CLASSES] = {0, ORDER_CAP_WORDS, 64, 32, 16, 0};
 
@@ -196,6 +195,8 @@ struct Settings {
     int band_min = 16, band_max = 1024;
     int pk_group = 0;           /* packed kernels: least lanes per pair (a power of two up to 32), 64 or 128 (the
                                    warps of a two- or four-warp block), or 0 to pick by the model (pk_plan) */
+    int tb_coop = 8192;         /* checkpoint walks: the longest pairs that take 8 lanes, besides the queries of
+                                   127+ words (-1: none takes more than one) */
     int wc_big_group = 0;       /* lane group of the 127+ word launch: 0 = automatic (64 when it fits), 32 or 64 */
     int wait_spins = 1 << 22;   /* polls of a wait between warps before it gives up (0.2 s or so) */
     int ksw_groups = 1;         /* unbanded ksw pairs of at most 31 query words run 4 to a warp (lane groups) */
