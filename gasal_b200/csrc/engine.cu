@@ -258,6 +258,27 @@ static int pk_class_of(uint32_t qlen, uint32_t tlen)
     return 2 + (words < PK_CLASS_WORDS[2]) + (words < PK_CLASS_WORDS[3]) + (words < PK_CLASS_WORDS[4]);
 }
 
+/* The batch's extreme lengths.  With AVX2 (32-bit unsigned minima and maxima)
+ * the loop takes a sixth of the baseline instruction set's time. */
+struct Extremes {
+    uint32_t min_q, max_q, max_t, max_min;
+};
+static inline __attribute__((always_inline)) Extremes extremes_of(const uint32_t *q, const uint32_t *t, int n)
+{
+    uint32_t lo = 0xFFFFFFFFu, hi = 0, th = 0, m = 0;
+    for (int i = 0; i < n; i++) {
+        const uint32_t ql = q[i], tl = t[i], s = ql < tl ? ql : tl;
+        lo = ql < lo ? ql : lo, hi = ql > hi ? ql : hi;
+        th = tl > th ? tl : th, m = s > m ? s : m;
+    }
+    return {lo, hi, th, m};
+}
+static Extremes extremes(const uint32_t *q, const uint32_t *t, int n) { return extremes_of(q, t, n); }
+__attribute__((target("avx2"))) static Extremes extremes_avx2(const uint32_t *q, const uint32_t *t, int n)
+{
+    return extremes_of(q, t, n);
+}
+
 /* Whether the packed kernels take this batch, and with what shapes.  They run
  * LOCAL, GLOBAL and target-tail SEMI_GLOBAL pairs of every length: at 150 bp
  * and 250-5000 bp they do two cells per instruction where the one-thread and
@@ -272,22 +293,9 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
                          (cfg.algo == SEMI_GLOBAL_ && cfg.tail == TARGET_ && cfg.start != WITH_TB_);
     if (!algo_ok || !st.persistent || (cfg.second && cfg.algo != GLOBAL_) || !pk_scores_ok(cfg.algo, cfg.sc))
         return GB_OK;
-    PkLengths cl[PK_CLASSES];
-    uint32_t min_q = 0xFFFFFFFFu, max_q = 0;
-    const int stride = std::max(1, b.n / 512);
-    for (int i = 0, next = 0; i < b.n; i++) {
-        const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
-        PkLengths &c = cl[pk_class_of(ql, tl)];
-        c.n++;
-        c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl);
-        c.max_min = std::max(c.max_min, (std::min(ql, tl) + 7) & ~7u); /* bytes after the end may be bases, and score */
-        min_q = std::min(min_q, ql), max_q = std::max(max_q, ql);
-        if (i >= next && c.ns < 128) {
-            next += stride;
-            c.qw[c.ns] = (int)((ql + 7) >> 3), c.tw[c.ns] = (int)((tl + 7) >> 3), c.ns++;
-        }
-    }
-    for (int c = 0; c < PK_CLASSES; c++) p.pk_all[c] = cl[c].n;
+    const Extremes x = __builtin_cpu_supports("avx2") ? extremes_avx2(b.h_q_len, b.h_t_len, b.n)
+                                                      : extremes(b.h_q_len, b.h_t_len, b.n);
+    const uint32_t min_q = x.min_q, max_q = x.max_q, max_t = x.max_t, max_min = x.max_min;
     /* An unordered batch is one class: equal lengths, or too few pairs for the order to matter.
      * Queries only are compared (the bound on a pair's lanes is its query; targets of any length
      * share a class).  The order's three launches cost 20 us; without it every pair has the lane
@@ -296,16 +304,35 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
      * 1,994 / 1,687, 1,000 1,712 / 3,195; GLOBAL of 50-1,000 bp, 100 pairs 256 / 225, 1,000
      * 306 / 323: the lines meet at about 300 pairs. */
     const bool order = b.n >= st.min_order_pairs || (b.n > 64 && st.min_order_pairs <= (1 << 29) && max_q > min_q + min_q / 2);
-    if (!order) {
-        PkLengths &z = cl[0];
-        for (int c = 1; c < PK_CLASSES; c++) {
-            z.n += cl[c].n;
-            z.max_q = std::max(z.max_q, cl[c].max_q), z.max_t = std::max(z.max_t, cl[c].max_t);
-            z.max_min = std::max(z.max_min, cl[c].max_min);
-            for (int k = 0; k < cl[c].ns && z.ns < 128; k++, z.ns++) z.qw[z.ns] = cl[c].qw[k], z.tw[z.ns] = cl[c].tw[k];
-            cl[c].n = cl[c].ns = 0;
+    PkLengths cl[PK_CLASSES];
+    auto add = [&](PkLengths &c, int i) {
+        c.qw[c.ns] = (int)((b.h_q_len[i] + 7) >> 3), c.tw[c.ns] = (int)((b.h_t_len[i] + 7) >> 3), c.ns++;
+    };
+    const int first = pk_class_of(max_q, max_t);
+    if (!order || (first > 1 && first == pk_class_of(min_q, 0))) {
+        /* every pair in one class: no look at each (300k pairs of 8-64 bases: 830 us a call with one) */
+        PkLengths &c = cl[order ? first : 0];
+        c.n = p.pk_all[order ? first : 0] = b.n;
+        c.max_q = max_q, c.max_t = max_t, c.max_min = max_min;
+        const int stride = std::max(1, b.n / 128);
+        for (int i = 0; i < b.n && c.ns < 128; i += stride) add(c, i);
+    } else {
+        const int stride = std::max(1, b.n / 512);
+        for (int i = 0, next = 0; i < b.n; i++) {
+            const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
+            PkLengths &c = cl[pk_class_of(ql, tl)];
+            c.n++;
+            c.max_q = std::max(c.max_q, ql), c.max_t = std::max(c.max_t, tl);
+            c.max_min = std::max(c.max_min, std::min(ql, tl));
+            if (i >= next && c.ns < 128) {
+                next += stride;
+                add(c, i);
+            }
         }
+        for (int c = 0; c < PK_CLASSES; c++) p.pk_all[c] = cl[c].n;
     }
+    /* whole words: bytes after the end may be bases, and score */
+    for (PkLengths &c : cl) c.max_min = (c.max_min + 7) & ~7u;
     p.pk_wc = false;
     for (int c = 0; c < PK_CLASSES; c++) {
         if (cl[c].n == 0) continue;
@@ -616,33 +643,39 @@ static int plan_batch_with(bool packed, const RunCfg &cfg, const DevBatch &b, co
         return GB_ERR_CUDA;
     /* tile budget: the setting, but at most half of the device memory that is
      * free or already held as this stream's tiles (fewer, longer chunks on a
-     * large device; room left for other streams) */
-    uint64_t budget_bytes = st.tb_budget_bytes, all = 0;
-    for (int i = 0; i < b.n; i++) all += tb_tiles(b.h_q_len[i], b.h_t_len[i]);
-    if (all > ws.tb_cap) { /* a batch that fits what is held needs no look at the device's memory */
+     * large device; room left for other streams).  A batch that fits what is
+     * held needs no look at the device's memory. */
+    uint64_t chunk_max = 0, all = 0;
+    auto lay_out = [&](uint64_t budget_bytes) {
+        const uint64_t budget = std::max<uint64_t>(budget_bytes / 16, 1);
+        p.cut = {0};
+        uint64_t run = 0;
+        chunk_max = all = 0;
+        for (int i = 0; i < b.n; i++) {
+            const uint64_t t = tb_tiles(b.h_q_len[i], b.h_t_len[i]);
+            if (run > 0 && run + t > budget) {
+                chunk_max = std::max(chunk_max, run);
+                all += run;
+                p.cut.push_back(i);
+                run = 0;
+            }
+            ws.h_tb_off[i] = run;
+            run += t;
+        }
+        chunk_max = std::max(chunk_max, run);
+        all += run;
+        p.cut.push_back(b.n);
+    };
+    lay_out(st.tb_budget_bytes);
+    if (all > ws.tb_cap) {
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-            const uint64_t avail = ((uint64_t)free_b + (uint64_t)ws.tb_cap * 16) / 2;
-            budget_bytes = std::min<uint64_t>(budget_bytes, std::max<uint64_t>(avail, (uint64_t)1 << 30));
+            const uint64_t avail = std::max<uint64_t>(((uint64_t)free_b + (uint64_t)ws.tb_cap * 16) / 2, (uint64_t)1 << 30);
+            if (avail < st.tb_budget_bytes && chunk_max > avail / 16) lay_out(avail);
         } else {
             cudaGetLastError();
         }
     }
-    const uint64_t budget = std::max<uint64_t>(budget_bytes / 16, 1);
-    p.cut = {0};
-    uint64_t run = 0, chunk_max = 0;
-    for (int i = 0; i < b.n; i++) {
-        const uint64_t t = tb_tiles(b.h_q_len[i], b.h_t_len[i]);
-        if (run > 0 && run + t > budget) {
-            chunk_max = std::max(chunk_max, run);
-            p.cut.push_back(i);
-            run = 0;
-        }
-        ws.h_tb_off[i] = run;
-        run += t;
-    }
-    chunk_max = std::max(chunk_max, run);
-    p.cut.push_back(b.n);
     if (grow((void **)&ws.tb, &ws.tb_cap, chunk_max, sizeof(uint4)) != GB_OK) return GB_ERR_ALLOC;
     size_t max_chunk = 0;
     for (size_t c = 0; c + 1 < p.cut.size(); c++) {

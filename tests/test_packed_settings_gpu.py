@@ -2,10 +2,11 @@
 the oracle's results, the warp-cooperative kernels' lane group leaves packed
 batches alone, the autotuner tries only what the batch's route uses, and a
 storage's graph is replayed for batches that differ in nothing the launches
-depend on."""
+depend on; and what the host spends on a large batch of short pairs."""
 import os
 import subprocess
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -124,3 +125,32 @@ def test_graph_replayed_for_an_unordered_batch_of_other_lengths():
                 assert np.array_equal(got[k], v), k
             seen.append({k: v - s0[k] for k, v in gl.graph_stats().items()})
     assert seen[0]["instantiated"] == 1 and seen[1]["relaunched"] == 1, seen
+
+
+def test_host_time_of_many_short_pairs():
+    """Planning 300,000 pairs of one class costs the host no more than twice the
+    plain form's (a look at each pair cost four times as much and set the time
+    of the call)."""
+    torch = pytest.importorskip("torch")
+    p = Params(algo=LOCAL)
+    rng = np.random.default_rng(8)
+    n, w = 300000, 40
+    seqs = rng.choice(np.frombuffer(b"ACGT", np.uint8), n * w)
+    off, ln = np.arange(n, dtype=np.uint32) * np.uint32(w), np.full(n, w, np.uint32)
+    b = Batch(seqs, seqs.copy(), off, off.copy(), ln, ln.copy())
+    m, keep, outs = _device(torch, p, b)
+    s = torch.cuda.current_stream().cuda_stream
+    saved, best = gl.get_tuning(), {}
+    try:
+        for persistent in (1, 0):
+            gl.set_tuning(persistent=persistent)
+            ts = []
+            for _ in range(12):
+                torch.cuda.synchronize()
+                t0 = time.perf_counter()
+                gl.align_dev(p, m, b.q_len, b.t_len, s)
+                ts.append(time.perf_counter() - t0)
+            best[persistent] = min(ts[2:])
+    finally:
+        gl.set_tuning(**saved)
+    assert best[1] < 2 * best[0], best
