@@ -126,8 +126,8 @@ static double steps_of(int g, int qw, int nb)
 /* Lane group of each class, block and grid.  Narrow groups waste fewer
  * lane-steps on fill, drain and the last round; wide ones give each pair less
  * time and the chip more warps, and hold fewer rings.  A class's narrowest
- * group is the one whose rings fit RING_WORDS per warp (14 of the 16 warps per
- * SM that registers allow).  From there the longest pairs' groups are widened
+ * group is the one whose rings fit RING_WORDS per warp (with the score table and
+ * the system's share 11 one-warp blocks per SM; registers allow 16 warps).  From there the longest pairs' groups are widened
  * -- to 32 lanes, or to the block's two or four warps -- until the launch's
  * modelled time, the larger of all warps' steps at the SMs' rate and any
  * class's longest pair, stops falling.  A step of one of A resident warps of
@@ -208,8 +208,9 @@ bool pk_plan(int algo, int start, const PkLengths *cl, int sms, int forced, PkPl
     p.cmp_q8[0] = (int)((max_q + 7) & ~7u), p.cmp_q8[1] = std::min(p.cmp_q8[0], PK_CMP_LONG);
     p.cmp_cols[0] = p.cmp_q8[0] >= PK_CMP_LONG ? ring_words(32, max_q) : 0;
     p.cmp_cols[1] = ring_words(4, (uint32_t)p.cmp_q8[1]);
-    const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1,
-                                   (size_t)std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]) * 4);
+    p.cmp_many = p.cmp_q8[0] <= PK_CMP_NARROW ? PK_CMP_MANY * sms : 0;
+    p.cmp_words = std::max(p.cmp_cols[0], (p.cmp_many ? 32 : 8) * p.cmp_cols[1]);
+    const int res = resident_warps(kernel_use(algo, PK_CMP, start), 1, (size_t)p.cmp_words * 4);
     p.cmp_blocks = std::min(p.cmp_cols[0] ? n : (n + 7) / 8, std::max(sms * res, sms));
     return res > 0;
 }
@@ -223,7 +224,7 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     cl.warp_words = p.warp_words;
     for (int c = 0; c < PK_CLASSES; c++) {
         if (n[c] == 0) continue;
-        cl.k[cl.n++] = {p.group[c], total, n[c], p.ring_cols[c], p.max_q8[c]};
+        cl.k[cl.n++] = {p.group[c], total, n[c], p.ring_cols[c], p.max_q8[c], 0};
         warps += ((long)n[c] * p.group[c] + 31) / 32;
         total += n[c];
     }
@@ -245,9 +246,9 @@ cudaError_t launch_dp_pk(int algo, int start, const DpArgs &a, const PkConst &pc
     DpArgs c = f;
     c.queue = wq + PK_CLASSES, c.defer = nullptr, c.ndefer = nullptr, c.n_dev = f.ndefer;
     PkClasses left;
-    left.warp_words = std::max(p.cmp_cols[0], 8 * p.cmp_cols[1]);
-    if (p.cmp_cols[0]) left.k[left.n++] = {32, 0, total, p.cmp_cols[0], p.cmp_q8[0]};
-    left.k[left.n++] = {4, 0, total, p.cmp_cols[1], p.cmp_q8[1]};
+    left.warp_words = p.cmp_words;
+    if (p.cmp_cols[0]) left.k[left.n++] = {32, 0, total, p.cmp_cols[0], p.cmp_q8[0], 0};
+    left.k[left.n++] = {4, 0, total, p.cmp_cols[1], p.cmp_q8[1], p.cmp_many};
     return launch(PK_CMP, c, left, defer, std::min(total, p.cmp_blocks), 1);
 }
 

@@ -739,6 +739,10 @@ __global__ void __launch_bounds__(32 * W, 16 / W)
             if (k.group == 32)
                 pk_pairs<32, 1, ALGO, START, FAST>(A, P, tab, mem, l + (A.n - 1), (int)A.n_dev[1], qu, k.ring_cols,
                                                     k.max_q8, -1);
+            else if (k.many > 0 && (int)A.n_dev[0] >= k.many)
+                pk_pairs<1, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols, k.max_q8);
+            else if (k.many > 0 && 5ll * (int)A.n_dev[0] >= k.many)
+                pk_pairs<2, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols, k.max_q8);
             else
                 pk_pairs<4, 1, ALGO, START, FAST>(A, P, tab, mem, l, (int)A.n_dev[0], qu, k.ring_cols, k.max_q8);
             continue;

@@ -37,6 +37,7 @@ constexpr int PK_FIFO = 32;
  * queries of up to max_q8 bases (in whole words). */
 struct PkClass {
     int32_t group, first, n, ring_cols, max_q8;
+    int32_t many; /* compare scoring: from this many pairs on one lane each, from a fifth two (0: never) */
 };
 constexpr int PK_CLASSES = 6;
 struct PkClasses {
@@ -45,9 +46,17 @@ struct PkClasses {
 };
 
 using PkKernel = void (*)(DpArgs, PkConst, PkClasses, const uint32_t *);
-/* compare scoring takes queries of PK_CMP_LONG bases on 32 lanes, shorter ones
- * on 4 (100k SEMI_GLOBAL 150 bp pairs with such targets: 8 lanes 4.1 ms) */
-constexpr int PK_CMP_LONG = 64 * 8;
+/* Compare scoring takes queries of PK_CMP_LONG bases on 32 lanes, shorter ones
+ * on 4 (100k SEMI_GLOBAL 150 bp pairs with such targets: 8 lanes 4.1 ms).  Where
+ * no query has more than PK_CMP_NARROW bases (32 rings of a warp then leave room
+ * for 11 warps an SM), many pairs take fewer: 4 lanes are 8 virtual ones, more
+ * than such a query's words or its rest of bands.  The kernel counts what is
+ * left to it: from PK_CMP_MANY pairs an SM 1 lane, from a fifth of that 2.
+ * LOCAL, us a call on 4 lanes / 1: 8k pairs 33 x 40 bases 57 / 68, 100 x 130
+ * 129 / 298, 20 x 2,000 664 / 919; 40k 135 / 101, 409 / 528, 2,495 / 1,686; 60k
+ * 175 / 103, 564 / 526, 3,519 / 1,703; 300k 692 / 309, 2,682 / 1,920, 17,190 /
+ * 6,730. */
+constexpr int PK_CMP_LONG = 64 * 8, PK_CMP_NARROW = 128, PK_CMP_MANY = 272;
 /* compare scoring; table scoring in blocks of 1, 2, 4 warps */
 enum PkVariant { PK_CMP, PK_W1, PK_W2, PK_W4, PK_VARIANTS };
 PkKernel pk_kernel_local(PkVariant v, int start);
@@ -68,7 +77,7 @@ struct PkPlan {
     int ring_cols[PK_CLASSES] = {}, max_q8[PK_CLASSES] = {};
     int warp_words = 0, warps = 0, blocks = 0;         /* blocks: most that are resident */
     /* compare scoring: long pairs (32 lanes), short ones (4) */
-    int cmp_cols[2] = {}, cmp_q8[2] = {}, cmp_blocks = 0;
+    int cmp_cols[2] = {}, cmp_q8[2] = {}, cmp_many = 0, cmp_words = 0, cmp_blocks = 0;
 };
 
 /* The packed kernels take LOCAL, GLOBAL and target-tail SEMI_GLOBAL without a

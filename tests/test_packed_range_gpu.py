@@ -1,7 +1,8 @@
 """The packed kernels at the edges of the values they accept: the longest pairs
 whose scores stay within 15 bits and the first that do not, bytes after a
 sequence's end that are bases (LOCAL scores them, as the reference does), and
-the lowest values of GLOBAL and SEMI_GLOBAL, against the oracle."""
+the lowest values of GLOBAL and SEMI_GLOBAL; and as many pairs with other codes as
+make compare scoring take two lanes each, or one.  Against the oracle."""
 from dataclasses import replace
 
 import numpy as np
@@ -65,3 +66,27 @@ def test_lowest_scores(p, e):
         for q in (1, 8, 500, 512, 513, 900):
             b = Batch.from_seqs([b"A" * q, b"C" * q], [b"C" * t, b"G" * t])
             _check(replace(p, **sc), b, f"{p.key()} {q} x {t}")
+
+
+@pytest.mark.parametrize("p", MODES, ids=lambda p: p.key())
+@pytest.mark.parametrize("n,longest", [(8200, 128), (40400, 128), (40400, 129)])
+def test_many_pairs_of_other_codes(p, n, longest):
+    """Pairs whose targets hold R, a fifth of 272 on each of 148 SMs and as many
+    as that, queries of 1 to 128 bases, or one of 129."""
+    rng = np.random.default_rng(longest)
+    w = 136
+    q = ACGT[rng.integers(0, 4, (n, w))]
+    t = q.copy()
+    m = rng.random((n, w)) < 0.05
+    t[m] = ACGT[rng.integers(0, 4, int(m.sum()))]
+    t[:, 0] = ord("R")
+    q[::7, 2] = ord("N")
+    t[::5, 3] = ord("N")
+    off = np.arange(n, dtype=np.uint32) * np.uint32(w)
+    ql = rng.integers(1, 129, n).astype(np.uint32)
+    tl = np.minimum(ql + rng.integers(0, 9, n).astype(np.uint32), 136)
+    tl[::9] = rng.integers(1, 137, len(tl[::9]))
+    ql[5] = longest
+    for x, ln in ((q, ql), (t, tl)):
+        x[np.arange(w)[None, :] >= ln[:, None]] = ord("N")
+    _check(p, Batch(q.reshape(-1), t.reshape(-1), off, off.copy(), ql, tl), p.key())

@@ -154,3 +154,35 @@ def test_host_time_of_many_short_pairs():
     finally:
         gl.set_tuning(**saved)
     assert best[1] < 2 * best[0], best
+
+
+def test_many_short_queries_of_other_codes_keep_the_plain_forms_time():
+    """100,000 pairs of 20-base queries whose targets hold R: compare scoring
+    on four lanes each took twice the plain form's time."""
+    torch = pytest.importorskip("torch")
+    p = Params(algo=LOCAL)
+    rng = np.random.default_rng(9)
+    n, q, t = 100000, 24, 1000
+    qs, ts = (rng.choice(np.frombuffer(b"ACGT", np.uint8), (n, w)) for w in (q, t))
+    ts[:, 0] = ord("R")
+    off = np.arange(n, dtype=np.uint32)
+    b = Batch(qs.reshape(-1), ts.reshape(-1), off * np.uint32(q), off * np.uint32(t), np.full(n, 20, np.uint32),
+              np.full(n, t, np.uint32))
+    m, keep, outs = _device(torch, p, b)
+    s = torch.cuda.current_stream().cuda_stream
+    saved, ms = gl.get_tuning(), {}
+    try:
+        for persistent in (1, 0):
+            gl.set_tuning(persistent=persistent)
+            for _ in range(3):
+                gl.align_dev(p, m, b.q_len, b.t_len, s)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(5):
+                gl.align_dev(p, m, b.q_len, b.t_len, s)
+            e1.record()
+            torch.cuda.synchronize()
+            ms[persistent] = e0.elapsed_time(e1)
+    finally:
+        gl.set_tuning(**saved)
+    assert ms[1] < 1.4 * ms[0], ms
