@@ -860,8 +860,9 @@ static int launch_ksw_split(const RunCfg &cfg, const DevBatch &b, const Plan &p,
         GB_CUDA(launch_ksw_wc(ra, ws.retry, n, p.ksw_slots, ws.fb, ws.queue + 2, ws.queue + 8, cells, s,
                               p.ksw_short > 0 ? -1 : -2, ws.queue + 11));
     } else {
-        /* a length order lists the short pairs last */
-        const int split = p.ksw_short <= 0 ? -2 : (order ? n - p.ksw_short : -1);
+        /* a length order lists the short pairs last; with nothing but short ones the lane groups
+         * take the whole list and the row kernels are not launched */
+        const int split = p.ksw_short <= 0 ? -2 : (order || p.ksw_short == n ? n - p.ksw_short : -1);
         GB_CUDA(launch_ksw_wc(p.a, order, n, p.ksw_slots, ws.fb, ws.queue + 2, ws.queue + 6, cells, s, split,
                               ws.queue + 10, ws.retry, ws.queue + 20));
     }

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 from gasal_b200 import lib as gl
-from gasal_b200.capi import Batch, Params, LOCAL, GLOBAL, SEMI_GLOBAL, WITH_START, WITH_TB, NONE, QUERY, TARGET, BOTH
+from gasal_b200.capi import Batch, Params, KSW, LOCAL, GLOBAL, SEMI_GLOBAL, WITH_START, WITH_TB, NONE, QUERY, TARGET, BOTH
 from oracle.bindings import oracle_align
 
 pytestmark = pytest.mark.gpu
@@ -93,3 +93,21 @@ def test_checkpoint_walks_by_lanes_per_pair(coop):
     r = subprocess.run([sys.executable, "-c", WALKS, ROOT], env=dict(os.environ, GASAL_B200_TB_COOP=str(coop)),
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("n", [3, 60, 2100])
+def test_ksw_batches_of_short_queries_only(n):
+    """Queries of at most 31 words alone: the lane groups take the whole list,
+    ordered or not, and hand seeds beyond 16 bits to the one-thread kernel."""
+    rng = np.random.default_rng(n)
+    qs = [ACGT[rng.integers(0, 4, int(k))] for k in rng.integers(1, 249, n)]
+    ts = [np.concatenate([q[:int(rng.integers(0, len(q) + 1))], ACGT[rng.integers(0, 4, int(rng.integers(0, 60)))]])
+          for q in qs]
+    b = Batch.from_seqs([q.tobytes() for q in qs], [t.tobytes() for t in ts])
+    b.seed = rng.integers(0, 100, n).astype(np.uint32)
+    b.seed[::3] = 33000
+    p = Params(algo=KSW, zdrop=50)
+    got, exp = gl.align(p, b).as_dict(p), oracle_align(p, b).as_dict(p)
+    for k, v in exp.items():
+        bad = np.nonzero(got[k] != v)[0]
+        assert not len(bad), f"{k}: {len(bad)} differ, first {bad[:5]} (q {b.q_len[bad[:5]]})"
