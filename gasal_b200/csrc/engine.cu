@@ -308,16 +308,14 @@ static int plan_pk(const RunCfg &cfg, const DevBatch &b, Workspace &ws, Plan &p,
     auto add = [&](PkLengths &c, int i) {
         c.qw[c.ns] = (int)((b.h_q_len[i] + 7) >> 3), c.tw[c.ns] = (int)((b.h_t_len[i] + 7) >> 3), c.ns++;
     };
-    const int first = pk_class_of(max_q, max_t);
+    const int first = pk_class_of(max_q, max_t), stride = std::max(1, b.n / 512);
     if (!order || (first > 1 && first == pk_class_of(min_q, 0))) {
         /* every pair in one class: no look at each (300k pairs of 8-64 bases: 830 us a call with one) */
         PkLengths &c = cl[order ? first : 0];
         c.n = p.pk_all[order ? first : 0] = b.n;
         c.max_q = max_q, c.max_t = max_t, c.max_min = max_min;
-        const int stride = std::max(1, b.n / 128);
         for (int i = 0; i < b.n && c.ns < 128; i += stride) add(c, i);
     } else {
-        const int stride = std::max(1, b.n / 512);
         for (int i = 0, next = 0; i < b.n; i++) {
             const uint32_t ql = b.h_q_len[i], tl = b.h_t_len[i];
             PkLengths &c = cl[pk_class_of(ql, tl)];
