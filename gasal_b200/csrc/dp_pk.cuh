@@ -39,16 +39,16 @@
  * waits are bounded: the warp votes after each, so one lane whose polls run out
  * ends the whole warp's sweep at the same step, and sets a word that the host
  * reports as an error (one lane polling for the warp through a shuffle instead
- * cost 100k LOCAL tracebacks of 50-5,000 bp 5%).  No warp waits in a circle: a round has at least as many steps as
- * the group virtual lanes, and the ring holds a whole one, so the last warp
- * never waits for room.
+ * cost 100k LOCAL tracebacks of 50-5,000 bp 5%).  No warp waits in a circle: a
+ * round has at least as many steps as the group virtual lanes, and the ring
+ * holds a whole one, so the last warp never waits for room.
  *
  * Measured on a B200 (us a batch, before with one pair per thread below 32
  * query words and one band per lane above, after): 300k SEMI_GLOBAL 150 bp with
  * starts 6,960 / 4,710; 200k LOCAL of 50-5,000 bp with starts 51,700 / 27,000;
  * 150k SEMI_GLOBAL of the same lengths 39,400 / 19,000; 100k GLOBAL of
  * 50-1,000 bp with traceback 19,000 / 6,400; 5k GLOBAL 150 bp 460 / 135; 1k
- * LOCAL of 250-2,000 bp 750,000 / 2,860.  Rates on equal lengths of 500: GLOBAL
+ * LOCAL of 250-2,000 bp 750,000 / 2,950.  Rates on equal lengths of 500: GLOBAL
  * 5.1 T cells/s, SEMI_GLOBAL 4.2, LOCAL 3.6.  A LOCAL step of a warp is about 700 instructions, 500 of
  * them on that pipe (73% busy at two warps a scheduler).
  *

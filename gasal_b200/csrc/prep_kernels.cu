@@ -32,7 +32,8 @@ __device__ __forceinline__ uint32_t pack8(uint32_t lo, uint32_t hi)
 
 /* One side's range, by the blocks [first, first + nblocks) of the launch: a
  * batch's queries and targets are packed by one launch (a second one was 3 of
- * the 120 us of a 64-pair call). */
+ * the 120 us of a 64-pair call); gb_align_dev_mixed still packs its sides one
+ * after the other. */
 struct PackSide {
     const uint8_t *ascii;
     uint32_t *words;

@@ -1,8 +1,10 @@
 /*
- * tb_kernel.cu -- traceback of the direction tiles into GASAL2's CIGAR bytes.
+ * tb_kernel.cu -- tracebacks into GASAL2's CIGAR bytes.
  *
- * Replaces reference src/kernels/get_tb.h:4-149.  One thread per pair walks
- * its tiles backwards.  Output format: one byte per run, (count << 2) | op
+ * Replaces reference src/kernels/get_tb.h:4-149.  traceback_kernel walks the
+ * direction tiles of the one-thread and warp-cooperative kernels, one thread per
+ * pair; traceback_points_kernel walks the packed kernels' checkpoints, one thread
+ * per pair or eight to the longest.  Output format: one byte per run, (count << 2) | op
  * with op 0 match, 1 mismatch, 2 deletion (consumes target), 3 insertion
  * (consumes query), count <= 63, written last operation first at the pair's
  * query offset of the device query batch; the run count replaces nothing else
